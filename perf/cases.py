@@ -170,8 +170,8 @@ def _operands(case, seed):
     if case["kind"] == "gate":  # a normalised state and a unitary
         d = math.isqrt(nb)
         a = _normal(gen, na, case["dtype"], math.sqrt(0.5 / na))
-        b = torch.linalg.qr(_normal(gen, nb, "complex128", 1.0).reshape(d, d))[0]
-        return a, b.contiguous().reshape(-1).to(a.dtype)
+        b = torch.from_numpy(_unitary(np.random.default_rng(seed), d).reshape(-1))
+        return a, b.to(DEVICE, a.dtype)
     scale = math.sqrt(0.5) * 2.0 ** -10
     return _normal(gen, na, case["dtype"], scale), _normal(gen, nb, case["dtype"], scale)
 
