@@ -15,11 +15,26 @@
 //
 // One CTA computes a 128 x 128 complex tile. Warp 0 lane 0 feeds a 3-stage
 // ring of shared-memory stages with TMA (8 boxes of 128 rows x 64 bytes,
-// 64-byte swizzle); warp 1 lane 0 issues tcgen05.mma (M=128, N=128, 32 bytes
-// of K per instruction: K=8 kind::tf32 or K=16 kind::f16) into one of two
-// TMEM accumulator sets (Cr, Ci: 2 x 256 columns) and releases stages with
+// 64-byte swizzle); warp 1 lane 0 issues tcgen05.mma (M=128, N=128 or 256, 32
+// bytes of K per instruction: K=8 kind::tf32 or K=16 kind::f16) into one of two
+// TMEM accumulator sets (2 x 256 columns) and releases stages with
 // tcgen05.commit; eight accumulator warps fold each finished K chunk into
 // FP32 registers (see the kernel comment) and write C.
+//
+// What bounds the product is the shared-memory port (128 bytes a clock): an
+// MMA of N = 128 reads 8 KB of operands in the 64 clocks it takes, the whole
+// port, and TMA writes the stages through the same port. N = 256 reads 12 KB
+// in 128 clocks. In the BF16 form the B planes lie in the stage as {Br_hi,
+// Bi_hi, Br_lo, Bi_lo}, so [Br; Bi] is one 256-row operand: Ar [Br; Bi] goes
+// into set 0 and Ai [Br; Bi] into set 1, all N = 256, 208 KB through the port
+// per 32 k instead of 256, and the fold adds (+, +) and (-, +), with half as
+// many terms per accumulator. Measured on M = 2^14, N = 2^12, K = 2^13, splits
+// included: 8.95 -> 8.20 ms at 4.5e-6 -> 4.4e-6 from FP64.
+// TF32 and FP16, the forms of whole networks, keep the N = 128 order: two sums
+// gave 6 % on a sliced 35-qubit amplitude but move its last bits, which
+// chunks, batches and resumed runs of one amplitude share; Ar [Br; Bi] as
+// N = 256 beside N = 128 for Ai (the same bits, 232 KB) measured no faster
+// there and 4 % slower on 2048 x 1024 x 1024.
 // The 3M ("Gauss") form uses three real products instead of four:
 //   P1 = Ar Br,  P2 = Ai Bi,  P3 = (Ar + Ai)(Br + Bi),
 //   Cr = P1 - P2,  Ci = P3 - P1 - P2,
@@ -61,8 +76,9 @@ constexpr int kTileRing = 4;                  // tile indices in flight between 
 //                 [-Bi, Br, Bi] (hi, lo); 6 MMAs of N = 256 per k step:
 //                 Ar [Br; Bi] -> [ArBr | ArBi] and Ai [-Bi; Br] ->
 //                 [-AiBi | AiBr] land on (Cr | Ci) in one instruction each.
-//  2 BF16 narrow: variant 0 on BF16 planes (kind::f16, 32 k per stage).
-//  4 FP16 narrow: variant 2 on FP16 planes of power-of-two scaled operands.
+//  2 BF16 narrow: the same stages of BF16 planes (kind::f16, 32 k per
+//                 stage); 6 MMAs of N = 256 per k step, two sets of sums.
+//  4 FP16 narrow: variant 0 on FP16 planes of power-of-two scaled operands.
 //  3 BF16 deep:   32-byte rows (16 k, 32-byte swizzle), 6 stages of 32 KB:
 //                 the same shared memory as variant 2 in twice as many,
 //                 half-size stages.
@@ -322,6 +338,21 @@ __device__ __forceinline__ void AddF32x2(float &a0, float &a1, float b0, float b
         : "f"(b0), "f"(b1));
 }
 
+// (a0, a1) += sign * (b0, b1), sign = 1 or -1: the product is exact, so this
+// rounds as an add or a subtraction does.
+__device__ __forceinline__ void SignedAddF32x2(float &a0, float &a1, float b0, float b1,
+                                               float sign)
+{
+    asm("{\n\t.reg .b64 pa, pb, ps;\n\t"
+        "mov.b64 pa, {%0, %1};\n\t"
+        "mov.b64 pb, {%2, %3};\n\t"
+        "mov.b64 ps, {%4, %4};\n\t"
+        "fma.rn.f32x2 pa, pb, ps, pa;\n\t"
+        "mov.b64 {%0, %1}, pa;\n\t}"
+        : "+f"(a0), "+f"(a1)
+        : "f"(b0), "f"(b1), "f"(sign));
+}
+
 __device__ __forceinline__ void TmemWaitLoad()
 {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -340,6 +371,9 @@ __device__ __forceinline__ void TmemWaitLoad()
 // Register budget: the ten warps spread over the SM's four register-file
 // partitions (16K registers each) three to a partition at most, so a thread
 // gets at most 168 registers (a few bytes of the epilogue spill).
+// BF16 (kTwoSums): set 0 holds Ar [Br; Bi] of the chunk, set 1 Ai [Br; Bi];
+// each is folded while the other's MMAs run, so a set is refilled half a
+// stage's MMA time after its last one.
 // 3M variants: three accumulators (P1, P2, P3) of 128 columns do not fit
 // twice in the 512 TMEM columns, so the products rotate through four
 // 128-column slots instead: product q = 3 g + p (stage g, product p) goes to
@@ -363,6 +397,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     constexpr int kAPlanes = kThreeM ? 6 : 4;
     constexpr int kFmt = Cfg::Fmt;
     constexpr bool kHalf = kFmt != kFmtTf32;
+    constexpr bool kTwoSums = kFmt == kFmtBf16 && !kWide && !kThreeM;
     constexpr int kBK = BlockK<V>();
     constexpr int kStages = Cfg::Stages;
     constexpr int kStageBytes = StageBytes<V>();
@@ -480,16 +515,18 @@ __global__ void __launch_bounds__(kThreads, 1)
                     else
                         TmaLoad3d(base + p * kTileBytes, &tmA, k0, m0, p, fb);
                 }
-                // B tiles: narrow {Br_hi, Br_lo, Bi_hi, Bi_lo}; wide
+                // B tiles: narrow {Br_hi, Br_lo, Bi_hi, Bi_lo}; two sums
+                // {Br_hi, Bi_hi, Br_lo, Bi_lo}; wide
                 // {-Bi_hi, Br_hi, Bi_hi, -Bi_lo, Br_lo, Bi_lo} (plane numbers
                 // 0 re_hi, 1 re_lo, 2 im_hi, 3 im_lo, 4 -im_hi, 5 -im_lo);
                 // 3M {Br_hi, Br_lo, Bi_hi, Bi_lo, Bs_hi, Bs_lo} (4, 5: re + im).
                 constexpr int kBTiles = Cfg::Tiles - kAPlanes;
 #pragma unroll
                 for (int t = 0; t < kBTiles; ++t) {
-                    const int plane = kWide ? (t == 0 ? 4 : t == 1 ? 0 : t == 2 ? 2
-                                               : t == 3 ? 5 : t == 4 ? 1 : 3)
-                                            : t;
+                    const int plane = kWide      ? (t == 0 ? 4 : t == 1 ? 0 : t == 2 ? 2
+                                                    : t == 3 ? 5 : t == 4 ? 1 : 3)
+                                      : kTwoSums ? (t & 1) * 2 + (t >> 1)
+                                                 : t;
                     if (b_batched)
                         TmaLoad4d(base + (kAPlanes + t) * kTileBytes, &tmB, k0, n0, bz, plane,
                                   fb);
@@ -558,6 +595,52 @@ __global__ void __launch_bounds__(kThreads, 1)
                     MmaCommit(SmemAddr(&acc_full[slot]));
                 }
                 MmaCommit(SmemAddr(&empty_bar[s]));
+            }
+            }
+            else if constexpr (kTwoSums) {
+            constexpr uint32_t kIdesc2 = InstrDesc(kBM, 2 * kBN, false, kFmt);
+            int in_chunk = 0;
+            for (int kt = 0; kt < ktiles && ok; ++kt) {
+                const long long gc = (long long)i * nchunks + kt / chunk_stages;
+                const bool chunk_start = in_chunk == 0;
+                const bool chunk_end = in_chunk == chunk_stages - 1 || kt == ktiles - 1;
+                in_chunk = chunk_end ? 0 : in_chunk + 1;
+                const long long g = (long long)i * ktiles + kt;
+                const int s = (int)(g % kStages);
+                if (!MbarWait(SmemAddr(&full_bar[s]), (uint32_t)(g / kStages) & 1u)) {
+                    ok = false;
+                    break;
+                }
+                FenceAfterSync();
+                const uint32_t base = SmemAddr(smem + s * kStageBytes);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) { // set 0: Ar [Br; Bi], set 1: Ai [Br; Bi]
+                    if (chunk_start) {
+                        if (!MbarWait(SmemAddr(&acc_empty[h]), ((uint32_t)gc & 1u) ^ 1u)) {
+                            ok = false;
+                            break;
+                        }
+                        FenceAfterSync();
+                    }
+                    const uint32_t d = tmem + h * 2 * kBN;
+#pragma unroll
+                    for (int kk = 0; kk < kRowBytes / 32; ++kk) {
+                        const uint32_t koff = kk * 32; // 32 bytes of K per MMA
+                        const uint64_t ah =
+                            SmemDesc<kRowBytes>(base + (2 * h) * kTileBytes + koff);
+                        const uint64_t al =
+                            SmemDesc<kRowBytes>(base + (2 * h + 1) * kTileBytes + koff);
+                        const uint64_t bh = SmemDesc<kRowBytes>(base + 4 * kTileBytes + koff);
+                        const uint64_t bl = SmemDesc<kRowBytes>(base + 6 * kTileBytes + koff);
+                        Mma<kHalf>(d, ah, bh, kIdesc2, (chunk_start && kk == 0) ? 0u : 1u);
+                        Mma<kHalf>(d, ah, bl, kIdesc2, 1u);
+                        Mma<kHalf>(d, al, bh, kIdesc2, 1u);
+                    }
+                    if (chunk_end)
+                        MmaCommit(SmemAddr(&acc_full[h]));
+                }
+                if (ok)
+                    MmaCommit(SmemAddr(&empty_bar[s]));
             }
             }
             else
@@ -729,6 +812,42 @@ __global__ void __launch_bounds__(kThreads, 1)
                                      SmemAddr(&acc_empty[slot]))
                                  : "memory");
             }
+        }
+        }
+        else if constexpr (kTwoSums) {
+        // Set 0 holds (Ar Br | Ar Bi), set 1 (Ai Br | Ai Bi):
+        // Cr += Ar Br, Ci += Ar Bi, then Cr -= Ai Bi, Ci += Ai Br.
+        uint32_t phase = (uint32_t)((long long)i * nchunks) & 1u;
+#pragma unroll 1
+        for (int q = 0; q < 2 * nchunks; ++q) {
+            const int h = q & 1;
+            ok = MbarWait(SmemAddr(&acc_full[h]), phase);
+            __syncwarp();
+            if (!ok)
+                break;
+            FenceAfterSync();
+            phase ^= (uint32_t)h;
+            const uint32_t col0 = tmem + lane_base + half * 64;
+            const uint32_t col_re = col0 + h * 3 * kBN, col_im = col0 + (1 + h) * kBN;
+            const float sign = h ? -1.f : 1.f;
+#pragma unroll
+            for (int c = 0; c < 64; c += 16) {
+                float re[16], im[16];
+                TmemLoad16(col_re + c, re);
+                TmemLoad16(col_im + c, im);
+                TmemWaitLoad();
+#pragma unroll
+                for (int j = 0; j < 16; j += 2) {
+                    SignedAddF32x2(acc_re[c + j], acc_re[c + j + 1], re[j], re[j + 1], sign);
+                    AddF32x2(acc_im[c + j], acc_im[c + j + 1], im[j], im[j + 1]);
+                }
+            }
+            FenceBeforeSync();
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(
+                                 SmemAddr(&acc_empty[h]))
+                             : "memory");
         }
         }
         else
