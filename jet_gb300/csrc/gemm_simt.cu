@@ -4,16 +4,16 @@
 // 128-168), which dispatches row-major CBLAS cgemm/zgemm (m, n > 1),
 // cgemv (right labels empty), cgemv^T (left labels empty) and cdotu (both
 // empty) with alpha = 1, beta = 0. Here:
-//  * gemm_kernel: 128x64 (complex64) / 64x64 (complex128) CTA tiles (32x64
-//    when M <= 32), 8-deep
-//    k slices staged in shared memory with register double buffering, each
-//    thread accumulating an 8x4 (4x4) block of complex outputs with 4 FMAs
-//    per complex multiply-add. Products whose tiles would leave SMs idle
-//    split k into partial sums in the workspace (GemmSplits), reduced in a
-//    fixed order.
+//  * gemm_kernel: CTA tiles of 64 x 64 down to 32 x 32 outputs by the shape
+//    (kTilesC64), k slices staged by cp.async, 4 FMAs per complex
+//    multiply-add. Products whose tiles would leave SMs idle split k into
+//    partial sums in the workspace (GemmSplits), reduced in a fixed order.
 //  * gemv_rows_kernel (n == 1) / gemv_cols_kernel (m == 1, also DOTU): split
 //    over k into partial sums, reduced in a fixed order by reduce_partials
 //    (deterministic).
+#include <algorithm>
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace jetgpu {
@@ -27,140 +27,189 @@ template <> struct C2<double> {
     using type = double2;
 };
 
-template <typename T> struct GemmCfg;
-template <> struct GemmCfg<float> {
-    static constexpr int TM = 8; // rows per thread
-};
-template <> struct GemmCfg<double> {
-    static constexpr int TM = 4;
+// Plain products, C = A B with FP32 or FP64 FMAs, k in increasing order per
+// output (re: +a.re b.re, -a.im b.im; im: +a.re b.im, +a.im b.re). Every
+// kernel and tile below runs that sequence, so the tile that a shape gets
+// never changes the result; only a split of k does.
+//
+// blockIdx.z = b * splits + s: batch b (operand strides sa, sb, 0 = shared;
+// C packed) and k range s (splits > 1: [s kchunk, (s + 1) kchunk), partial
+// sums to C + (s * batch + b) * M * N, reduced later). Tiles come in
+// row-major order over one grid dimension (N tiles fastest), so M may exceed
+// 65535 tiles (2^23 rows).
+template <typename V> struct GemmOperands {
+    const V *A, *B;
+    V *C;
+    int64_t M, N, K;   // this CTA's k extent
+    int64_t lda;       // A's row length (the whole k)
+    int64_t m0, n0;
 };
 
-constexpr int kBK = 8;
-constexpr int kTN = 4;
-constexpr int kTX = 16, kTY = 16; // 256 threads
-
-template <typename T, int TM>
-__global__ void __launch_bounds__(256)
-    gemm_kernel(const typename C2<T>::type *__restrict__ A,
-                const typename C2<T>::type *__restrict__ B,
-                typename C2<T>::type *__restrict__ C, int64_t M, int64_t N,
-                int64_t K, T scale, int64_t sa, int64_t sb, int splits, int64_t kchunk)
+template <typename V, int BM, int BN>
+__device__ __forceinline__ GemmOperands<V> GemmBlock(const V *A, const V *B, V *C, int64_t M,
+                                                     int64_t N, int64_t K, int64_t sa,
+                                                     int64_t sb, int splits, int64_t kchunk)
 {
-    using V = typename C2<T>::type;
-    // blockIdx.z = b * splits + s: batch b (operand strides sa, sb, 0 =
-    // shared; C packed) and k range s (splits > 1: [s kchunk, (s + 1)
-    // kchunk), partial sums to C + (s * batch + b) * M * N, reduced later).
     const int64_t s = (int64_t)blockIdx.z % splits;
     const int64_t bz = (int64_t)blockIdx.z / splits;
     const int64_t batch = (int64_t)gridDim.z / splits;
-    A += bz * sa;
-    B += bz * sb;
-    C += (s * batch + bz) * M * N;
-    const int64_t lda = K; // A's row length
     const int64_t k_begin = s * kchunk;
     const int64_t k_end = min(K, k_begin + kchunk);
-    A += k_begin;
-    B += k_begin * N;
-    K = k_end > k_begin ? k_end - k_begin : 0; // this split's k range
-    constexpr int BM = TM * kTY;
-    constexpr int BN = kTN * kTX;
-    constexpr int A_PER = BM * kBK / 256; // A elements loaded per thread
-    constexpr int B_PER = BN * kBK / 256;
-
-    __shared__ V As[2][kBK][BM + 1];
-    __shared__ V Bs[2][kBK][BN];
-
-    const int tid = threadIdx.x;
-    const int tx = tid % kTX, ty = tid / kTX;
-    // Tiles in row-major order over one grid dimension (N tiles fastest), so
-    // M may exceed 65535 tiles (2^23 rows).
     const int64_t tiles_n = (N + BN - 1) / BN;
-    const int64_t m0 = ((int64_t)blockIdx.x / tiles_n) * BM;
-    const int64_t n0 = ((int64_t)blockIdx.x % tiles_n) * BN;
+    GemmOperands<V> o;
+    o.A = A + bz * sa + k_begin;
+    o.B = B + bz * sb + k_begin * N;
+    o.C = C + (s * batch + bz) * M * N;
+    o.M = M;
+    o.N = N;
+    o.K = k_end > k_begin ? k_end - k_begin : 0;
+    o.lda = K;
+    o.m0 = ((int64_t)blockIdx.x / tiles_n) * BM;
+    o.n0 = ((int64_t)blockIdx.x % tiles_n) * BN;
+    return o;
+}
 
-    V acc[TM][kTN];
+// One element by cp.async (zero-filled when !valid: nothing is read).
+template <typename V> __device__ __forceinline__ void CpAsyncElem(V *smem, const V *src, bool valid)
+{
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem);
+    const int n = valid ? (int)sizeof(V) : 0; // 0: zero-fill, nothing read
+    if constexpr (sizeof(V) == 8)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(n)
+                     : "memory");
+    else
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(n)
+                     : "memory");
+}
+
+// TX x TY threads, each a TM x TN block of outputs of a (TY TM) x (TX TN) tile.
+// The k slices arrive by cp.async through a ring of three stages, two in
+// flight, so a CTA alone on its SM does not wait out a memory latency per
+// slice (with one slice in registers and one in shared memory that took 2,400
+// clocks per 8 k). A thread's rows and columns come in adjacent pairs
+// (complex64), so each shared-memory load brings two elements.
+// complex64 is bound by FMA issue: the register file feeds about 70 % of the
+// FMA pipe (56 TFLOP/s of 80) with three-operand FMAs at this reuse; packed
+// FMAs (fma.rn.f32x2) measured 38, and larger tiles (128 x 64, 8 x 8 outputs a
+// thread) no more than 64 x 64 while wasting more of the last wave (2187 x
+// 2187 in 128 x 64 tiles is 2.07 waves).
+// complex128 is bound by the FP64 pipe (1.1 TFLOP/s), whatever the block: 32 x
+// 32 tiles waste least on edges and on the last wave. 900 x 770 x 515: 4.14 ->
+// 2.60 ms (64 x 64 tiles were 195 CTAs on 152 SMs, 15 % padding).
+template <typename T, int TM, int TN, int TX, int TY, int BK, int kMinBlocks>
+__global__ void __launch_bounds__(TX *TY, kMinBlocks)
+    gemm_kernel(const typename C2<T>::type *__restrict__ A,
+                const typename C2<T>::type *__restrict__ B,
+                typename C2<T>::type *__restrict__ C, int64_t M, int64_t N, int64_t K, T scale,
+                int64_t sa, int64_t sb, int splits, int64_t kchunk)
+{
+    using V = typename C2<T>::type;
+    constexpr int kThreads = TX * TY, BM = TY * TM, BN = TX * TN, NS = 3;
+    constexpr int G = 16 / sizeof(V); // adjacent rows (columns) per thread and load
+    static_assert(TM % G == 0 && TN % G == 0, "whole pairs");
+    static_assert(BM * BK % kThreads == 0 && BN * BK % kThreads == 0, "whole loads");
+    struct alignas(16) Pack {
+        V v[G];
+    };
+    __shared__ __align__(16) V As[NS][BK][BM + G];
+    __shared__ __align__(16) V Bs[NS][BK][BN];
+    const auto o = GemmBlock<V, BM, BN>(A, B, C, M, N, K, sa, sb, splits, kchunk);
+    const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+
+    auto load = [&](int st, int64_t t) {
+        const int64_t k0 = t * BK;
+#pragma unroll
+        for (int q = 0; q < BM * BK / kThreads; ++q) {
+            const int e = tid + kThreads * q, row = e / BK, col = e % BK;
+            const bool ok = o.m0 + row < o.M && k0 + col < o.K;
+            CpAsyncElem(&As[st][col][row], ok ? o.A + (o.m0 + row) * o.lda + k0 + col : A, ok);
+        }
+#pragma unroll
+        for (int q = 0; q < BN * BK / kThreads; ++q) {
+            const int e = tid + kThreads * q, row = e / BN, col = e % BN;
+            const bool ok = k0 + row < o.K && o.n0 + col < o.N;
+            CpAsyncElem(&Bs[st][row][col], ok ? o.B + (k0 + row) * o.N + o.n0 + col : B, ok);
+        }
+    };
+
+    V acc[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < kTN; ++j)
+        for (int j = 0; j < TN; ++j)
             acc[i][j] = V{0, 0};
-
-    V ra[A_PER], rb[B_PER];
-    auto load_tiles = [&](int64_t k0) {
+    const int64_t ktiles = (o.K + BK - 1) / BK;
+    // Every iteration commits one group (empty past the last slice), so
+    // wait_group NS - 2 always means "slice t has landed".
 #pragma unroll
-        for (int q = 0; q < A_PER; ++q) {
-            int row = tid / kBK + q * (256 / kBK);
-            int col = tid % kBK;
-            int64_t gm = m0 + row, gk = k0 + col;
-            ra[q] = (gm < M && gk < K) ? A[gm * lda + gk] : V{0, 0};
-        }
-#pragma unroll
-        for (int q = 0; q < B_PER; ++q) {
-            int row = tid / BN + q * (256 / BN);
-            int col = tid % BN;
-            int64_t gk = k0 + row, gn = n0 + col;
-            rb[q] = (gk < K && gn < N) ? B[gk * N + gn] : V{0, 0};
-        }
-    };
-    auto store_tiles = [&](int buf) {
-#pragma unroll
-        for (int q = 0; q < A_PER; ++q) {
-            int row = tid / kBK + q * (256 / kBK);
-            int col = tid % kBK;
-            As[buf][col][row] = ra[q];
-        }
-#pragma unroll
-        for (int q = 0; q < B_PER; ++q) {
-            int row = tid / BN + q * (256 / BN);
-            int col = tid % BN;
-            Bs[buf][row][col] = rb[q];
-        }
-    };
-
-    const int64_t ktiles = (K + kBK - 1) / kBK;
-    if (ktiles > 0) {
-        load_tiles(0);
-        store_tiles(0);
+    for (int q = 0; q < NS - 1; ++q) {
+        if (q < ktiles)
+            load(q, q);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
-    __syncthreads();
-    for (int64_t kt = 0; kt < ktiles; ++kt) {
-        const int buf = kt & 1;
-        const bool more = kt + 1 < ktiles;
-        if (more)
-            load_tiles((kt + 1) * kBK);
+    int st = 0;
+    for (int64_t t = 0; t < ktiles; ++t) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(NS - 2) : "memory");
+        __syncthreads(); // slice t is visible, and slice t - 1 has been read
+        if (t + NS - 1 < ktiles)
+            load(st == 0 ? NS - 1 : st - 1, t + NS - 1);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
 #pragma unroll
-        for (int k = 0; k < kBK; ++k) {
-            V a[TM], b[kTN];
+        for (int k = 0; k < BK; ++k) {
+            V a[TM], b[TN];
 #pragma unroll
-            for (int i = 0; i < TM; ++i)
-                a[i] = As[buf][k][ty + kTY * i];
+            for (int i = 0; i < TM; i += G) {
+                const Pack w = *reinterpret_cast<const Pack *>(&As[st][k][G * ty + TY * i]);
 #pragma unroll
-            for (int j = 0; j < kTN; ++j)
-                b[j] = Bs[buf][k][tx + kTX * j];
+                for (int u = 0; u < G; ++u)
+                    a[i + u] = w.v[u];
+            }
 #pragma unroll
-            for (int i = 0; i < TM; ++i)
+            for (int j = 0; j < TN; j += G) {
+                const Pack w = *reinterpret_cast<const Pack *>(&Bs[st][k][G * tx + TX * j]);
 #pragma unroll
-                for (int j = 0; j < kTN; ++j) {
+                for (int u = 0; u < G; ++u)
+                    b[j + u] = w.v[u];
+            }
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
                     acc[i][j].x = fma(a[i].x, b[j].x, acc[i][j].x);
-                    acc[i][j].x = fma(-a[i].y, b[j].y, acc[i][j].x);
                     acc[i][j].y = fma(a[i].x, b[j].y, acc[i][j].y);
+                }
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
+                    acc[i][j].x = fma(-a[i].y, b[j].y, acc[i][j].x);
                     acc[i][j].y = fma(a[i].y, b[j].x, acc[i][j].y);
                 }
+            }
         }
-        if (more)
-            store_tiles(buf ^ 1);
-        __syncthreads();
+        st = st + 1 == NS ? 0 : st + 1;
     }
+    // Whole 16-byte pairs where C's rows allow it.
+    const bool vec = o.N % G == 0 && (reinterpret_cast<uintptr_t>(o.C) & 15) == 0;
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
-        int64_t gm = m0 + ty + kTY * i;
-        if (gm >= M)
+        const int64_t gm = o.m0 + G * ty + TY * (i - i % G) + i % G;
+        if (gm >= o.M)
             continue;
 #pragma unroll
-        for (int j = 0; j < kTN; ++j) {
-            int64_t gn = n0 + tx + kTX * j;
-            if (gn < N)
-                C[gm * N + gn] = V{acc[i][j].x * scale, acc[i][j].y * scale};
+        for (int j = 0; j < TN; j += G) {
+            const int64_t gn = o.n0 + G * tx + TX * j;
+            Pack w;
+#pragma unroll
+            for (int u = 0; u < G; ++u)
+                w.v[u] = V{acc[i][j + u].x * scale, acc[i][j + u].y * scale};
+            if (vec) {
+                if (gn < o.N)
+                    *reinterpret_cast<Pack *>(o.C + gm * o.N + gn) = w;
+                continue;
+            }
+#pragma unroll
+            for (int u = 0; u < G; ++u)
+                if (gn + u < o.N)
+                    o.C[gm * o.N + gn + u] = w.v[u];
         }
     }
 }
@@ -341,18 +390,6 @@ __global__ void __launch_bounds__(256)
 //    (MT / 4) x (NT / 8) block, so each warp covers the whole output;
 //  * the warps' sums are added in warp order in shared memory and the k
 //    ranges' in the workspace by reduce_partials: a fixed order.
-template <typename V> __device__ __forceinline__ void CpAsyncElem(V *smem, const V *src, bool valid)
-{
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem);
-    const int n = valid ? (int)sizeof(V) : 0; // 0: zero-fill, nothing read
-    if constexpr (sizeof(V) == 8)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(n)
-                     : "memory");
-    else
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(n)
-                     : "memory");
-}
-
 template <typename T, int MT, int NT>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
     gemm_small_kernel(const typename C2<T>::type *__restrict__ A,
@@ -575,17 +612,55 @@ int64_t SmallSplits(int64_t batch, int64_t K, int64_t out_bytes, size_t elem_byt
     return s < 2 ? 1 : s;
 }
 
-// Rows per thread of the SIMT product: the full 128 (complex64) / 64
-// (complex128) row tiles, or 32-row tiles when M is at most 32 (skinny
-// products would leave most of a full tile empty).
-template <typename T> inline int GemmTM(int64_t M) { return M <= 32 ? 2 : GemmCfg<T>::TM; }
+// The tiles of the matrix product and the measured clocks that one k of a tile
+// takes: in a CTA alone on its SM, and as its share of a full SM. A launch
+// takes the tile whose busiest SM finishes first: large products 64 x 64, or
+// 64 x 32 of 64 threads where 64 x 64 would leave the last wave thin; products
+// of few tiles the smaller blocks, whose CTAs finish sooner. Measured against
+// 128 x 64 tiles alone: 2187 x 2187 x 729 713 -> 568 us, 512 x 32 x 512 55 ->
+// 14, 9 x (81 x 243 x 243) 52 -> 17, 16 x (1024 x 8192 x 16) 456 -> 438, 4096 x
+// 4096 x 1024 2,765 -> 2,450.
+struct GemmTile {
+    int bm, bn;
+    double alone, shared;
+};
+constexpr GemmTile kTilesC64[] = {
+    {64, 64, 215, 183}, // 8 x 4 a thread, 128 threads
+    {64, 64, 199, 188}, // 4 x 4, 256 threads
+    {64, 32, 215, 97},  // 8 x 4, 64 threads
+    {64, 32, 122, 105}, // 4 x 2, 256 threads
+    {32, 64, 128, 112}, // 2 x 4
+    {32, 32, 83, 61},   // 2 x 2
+};
+constexpr int kNumTilesC64 = sizeof(kTilesC64) / sizeof(kTilesC64[0]);
+constexpr GemmTile kTileC128 = {32, 32, 0, 0};
 
-template <typename T> inline void GemmGrid(int64_t M, int64_t N, int64_t &tiles_n, int64_t &tiles_m)
+inline int64_t CeilDiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
+// Clocks per k on the busiest SM of a launch over `z` products of M x N.
+inline double TileClocks(const GemmTile &t, int64_t M, int64_t N, int64_t z)
 {
-    const int BM = GemmTM<T>(M) * kTY;
-    constexpr int BN = kTN * kTX;
-    tiles_n = (N + BN - 1) / BN;
-    tiles_m = (M + BM - 1) / BM;
+    const int64_t per_sm = CeilDiv(CeilDiv(M, t.bm) * CeilDiv(N, t.bn) * z, SmCount());
+    return std::max(t.alone, (double)per_sm * t.shared);
+}
+
+inline int PickTileC64(int64_t M, int64_t N, int64_t z)
+{
+    int best = 0;
+    for (int i = 1; i < kNumTilesC64; ++i)
+        if (TileClocks(kTilesC64[i], M, N, z) < TileClocks(kTilesC64[best], M, N, z))
+            best = i;
+    return best;
+}
+
+// Split-k factor of a batched product (fixed: the slices of a sliced network
+// keep their bits whatever tile a launch gets): GemmSplits over tiles of 128
+// (complex64) or 64 (complex128) rows, 32 when M <= 32, and 64 columns.
+template <typename T> int64_t BatchedSplits(int64_t batch, int64_t M, int64_t N, int64_t K)
+{
+    const int64_t bm = M <= 32 ? 32 : (sizeof(T) == 4 ? 128 : 64);
+    return GemmSplits(CeilDiv(M, bm) * CeilDiv(N, 64) * batch, batch, K,
+                      batch * M * N * (int64_t)(2 * sizeof(T)));
 }
 
 // Split-k factor for the vector kernels: enough CTAs to fill the GPU, with at
@@ -640,10 +715,8 @@ size_t VectorWorkspace(int64_t batch, int64_t m, int64_t n, int64_t k)
                 SmallSplits(batch, k, batch * m * n * (int64_t)sizeof(V), sizeof(V));
             return S > 1 ? (size_t)(S * batch * m * n) * sizeof(V) : 0;
         }
-        // Matrix products: partial sums of the k splits (GemmSplits).
-        int64_t tn, tm;
-        GemmGrid<T>(m, n, tn, tm);
-        const int64_t S = GemmSplits(tn * tm * batch, batch, k, batch * m * n * (int64_t)sizeof(V));
+        // Matrix products: partial sums of the k splits.
+        const int64_t S = BatchedSplits<T>(batch, m, n, k);
         return S > 1 ? (size_t)(S * batch * m * n) * sizeof(V) : 0;
     }
     int64_t blocks, len;
@@ -717,23 +790,43 @@ int GemmT(const typename C2<T>::type *A, const typename C2<T>::type *B, typename
             return rc;
         return ReducePartials<T>(dst, C, batch * M * N, S, stream);
     }
-    int64_t tn, tm;
-    GemmGrid<T>(M, N, tn, tm);
-    const int64_t S =
-        (need > 0 && ws != nullptr && ws_bytes >= need)
-            ? GemmSplits(tn * tm * batch, batch, K, batch * M * N * (int64_t)sizeof(V))
-            : 1;
+    const int64_t S = (need > 0 && ws != nullptr && ws_bytes >= need)
+                          ? BatchedSplits<T>(batch, M, N, K)
+                          : 1;
     const int64_t kchunk = (K + S - 1) / S;
-    JETGPU_REQUIRE(tn * tm <= 0x7fffffffLL && batch * S <= 65535,
-                   "product too large for one launch");
-    const dim3 grid((unsigned)(tn * tm), 1u, (unsigned)(batch * S));
+    const int tile = sizeof(T) == 4 ? PickTileC64(M, N, batch * S) : 0;
+    const GemmTile t = sizeof(T) == 4 ? kTilesC64[tile] : kTileC128;
+    const int64_t tiles = CeilDiv(M, t.bm) * CeilDiv(N, t.bn);
+    JETGPU_REQUIRE(tiles <= 0x7fffffffLL && batch * S <= 65535, "product too large for one launch");
+    const dim3 grid((unsigned)tiles, 1u, (unsigned)(batch * S));
     V *dst = S > 1 ? (V *)ws : C;
-    if (GemmTM<T>(M) == 2)
-        gemm_kernel<T, 2><<<grid, 256, 0, stream>>>(A, B, dst, M, N, K, scale, sa, sb, (int)S,
-                                                    kchunk);
-    else
-        gemm_kernel<T, GemmCfg<T>::TM><<<grid, 256, 0, stream>>>(A, B, dst, M, N, K, scale, sa,
-                                                                 sb, (int)S, kchunk);
+    const auto launch = [&](auto kernel, int threads) {
+        kernel<<<grid, threads, 0, stream>>>(A, B, dst, M, N, K, scale, sa, sb, (int)S, kchunk);
+    };
+    if constexpr (std::is_same<T, double>::value) {
+        launch(gemm_kernel<double, 2, 2, 16, 16, 8, 1>, 256);
+    }
+    else {
+        switch (tile) {
+        case 0:
+            launch(gemm_kernel<float, 8, 4, 16, 8, 8, 3>, 128);
+            break;
+        case 1:
+            launch(gemm_kernel<float, 4, 4, 16, 16, 16, 2>, 256);
+            break;
+        case 2:
+            launch(gemm_kernel<float, 8, 4, 8, 8, 8, 6>, 64);
+            break;
+        case 3:
+            launch(gemm_kernel<float, 4, 2, 16, 16, 16, 2>, 256);
+            break;
+        case 4:
+            launch(gemm_kernel<float, 2, 4, 16, 16, 16, 2>, 256);
+            break;
+        default:
+            launch(gemm_kernel<float, 2, 2, 16, 16, 16, 3>, 256);
+        }
+    }
     int rc = CheckLaunch("gemm_kernel");
     if (rc || S == 1)
         return rc;
