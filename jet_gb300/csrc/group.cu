@@ -12,9 +12,18 @@
 // the batch axes is absorbed into the load. C is written packed, batch x m x
 // n, row-major, as jetgpu_contract_batched writes it.
 //
-// CTA tiles are 32 x 32 outputs of one (task, batch item); 256 threads, each
-// accumulating 2 x 2 complex outputs in the element type (FP32 or FP64 FMA,
-// the plain form's arithmetic) over k slices of 32 staged in shared memory.
+// CTA tiles are 32 x 32 outputs of one (task, batch item), 256 threads, FP32
+// or FP64 FMAs over k in order (the plain form's arithmetic).
+//
+// Bound by latency: the tasks of a circuit network are a few outputs over a
+// few k (2 x 2 x 8), and a level's launch is a chain of dependent loads (task,
+// offset tables, elements). A tile of little work (kFlatWork) gives one output
+// to each thread, which reads its k values straight through the tables with
+// all loads of eight k issued before any arithmetic: no staging, no barrier.
+// Through staged 32 x 32 x 32 slices, mostly padding, the smallest launch took
+// 7.5 us. Tiles of more work are staged in shared memory, 2 x 2 outputs a
+// thread. The launch uses programmatic stream serialisation, so that a chain
+// of levels overlaps each launch with the end of the one before.
 #include "common.cuh"
 
 namespace jetgpu {
@@ -34,6 +43,19 @@ template <> struct V2<double> {
     using type = double2;
 };
 
+// Most multiply-adds of a tile that goes through the tables directly (8 k of a
+// full 32 x 32 tile), and its longest k.
+constexpr uint64_t kFlatWork = 8192;
+constexpr uint64_t kFlatK = 64;
+
+template <typename V> __device__ __forceinline__ void GroupMac(V &acc, const V &a, const V &b)
+{
+    acc.x = fma(a.x, b.x, acc.x);
+    acc.x = fma(-a.y, b.y, acc.x);
+    acc.y = fma(a.x, b.y, acc.y);
+    acc.y = fma(a.y, b.x, acc.y);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kGThreads)
     group_contract_kernel(const jetgpu_group_task *__restrict__ tasks, int n_tasks,
@@ -41,34 +63,46 @@ __global__ void __launch_bounds__(kGThreads)
 {
     using V = typename V2<T>::type;
     __shared__ uint64_t first_tile[kMaxTasks + 1];
+    __shared__ uint64_t warp_sum[kGThreads / 32];
     __shared__ V As[kGK][kGT + 1];
     __shared__ V Bs[kGK][kGT + 1];
-    // First tile of every task: thread t reads task t's tile count, then a
-    // block-wide inclusive scan (kMaxTasks = blockDim.x = 256: 8 rounds).
-    // One thread walking the tasks took 0.13 us a task, 30 us for 184.
+    // Every memory access follows this wait for the kernel before; the next
+    // launch may start once every CTA is past it.
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // First tile of every task: thread t reads task t's tile count, then an
+    // inclusive scan by warps and over the eight warp sums.
     {
-        const int tid = threadIdx.x;
-        uint64_t mine = 0;
+        const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+        uint64_t sum = 0;
         if (tid < n_tasks) {
             const jetgpu_group_task &q = tasks[tid];
-            mine = q.batch * ((q.m + kGT - 1) / kGT) * ((q.n + kGT - 1) / kGT);
+            sum = q.batch * ((q.m + kGT - 1) / kGT) * ((q.n + kGT - 1) / kGT);
         }
-        first_tile[tid + 1] = mine;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint64_t add = __shfl_up_sync(0xffffffffu, sum, off);
+            if (lane >= off)
+                sum += add;
+        }
+        if (lane == 31)
+            warp_sum[warp] = sum;
+        __syncthreads();
+        for (int w = 0; w < warp; ++w)
+            sum += warp_sum[w];
+        first_tile[tid + 1] = sum;
         if (tid == 0)
             first_tile[0] = 0;
         __syncthreads();
-        for (int off = 1; off < kMaxTasks; off <<= 1) {
-            const uint64_t add = tid >= off ? first_tile[tid + 1 - off] : 0;
-            __syncthreads();
-            first_tile[tid + 1] += add;
-            __syncthreads();
-        }
     }
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16; // 2 x 2 outputs each
-    int t = 0; // this CTA's tiles come in increasing order: the task only advances
     for (uint64_t g = blockIdx.x; g < total_tiles; g += gridDim.x) {
-        while (t + 1 < n_tasks && first_tile[t + 1] <= g)
-            ++t;
+        // The last task whose first tile is at most g.
+        int t = 0;
+#pragma unroll
+        for (int step = kMaxTasks / 2; step > 0; step >>= 1)
+            if (t + step < n_tasks && first_tile[t + step] <= g)
+                t += step;
         const jetgpu_group_task &q = tasks[t];
         const uint64_t local = g - first_tile[t];
         const uint64_t tiles_n = (q.n + kGT - 1) / kGT;
@@ -78,6 +112,33 @@ __global__ void __launch_bounds__(kGThreads)
         const uint64_t m0 = (r / tiles_n) * kGT, n0 = (r % tiles_n) * kGT;
         const V *A = static_cast<const V *>(q.A) + q.a_bat[b];
         const V *B = static_cast<const V *>(q.B) + q.b_bat[b];
+        V *C = static_cast<V *>(q.C) + b * q.m * q.n;
+        const uint32_t rows = (uint32_t)min(q.m - m0, (uint64_t)kGT);
+        const uint32_t cols = (uint32_t)min(q.n - n0, (uint64_t)kGT);
+        if (q.k <= kFlatK && rows * cols * q.k <= kFlatWork) {
+            const uint32_t k = (uint32_t)q.k;
+            for (uint32_t e = threadIdx.x; e < rows * cols; e += kGThreads) {
+                const uint32_t i = e / cols, j = e - i * cols;
+                const V *pa = A + q.a_row[m0 + i];
+                const V *pb = B + q.b_col[n0 + j];
+                V acc{0, 0};
+                for (uint32_t k0 = 0; k0 < k; k0 += 8) {
+                    V av[8], bv[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) { // past k: the last product's loads again
+                        const uint32_t kk = min(k0 + u, k - 1);
+                        av[u] = pa[q.a_col[kk]];
+                        bv[u] = pb[q.b_row[kk]];
+                    }
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                        if (k0 + u < k)
+                            GroupMac(acc, av[u], bv[u]);
+                }
+                C[(m0 + i) * q.n + n0 + j] = acc;
+            }
+            continue;
+        }
         V acc[2][2];
 #pragma unroll
         for (int i = 0; i < 2; ++i)
@@ -106,16 +167,11 @@ __global__ void __launch_bounds__(kGThreads)
 #pragma unroll
                 for (int i = 0; i < 2; ++i)
 #pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        acc[i][j].x = fma(av[i].x, bv[j].x, acc[i][j].x);
-                        acc[i][j].x = fma(-av[i].y, bv[j].y, acc[i][j].x);
-                        acc[i][j].y = fma(av[i].x, bv[j].y, acc[i][j].y);
-                        acc[i][j].y = fma(av[i].y, bv[j].x, acc[i][j].y);
-                    }
+                    for (int j = 0; j < 2; ++j)
+                        GroupMac(acc[i][j], av[i], bv[j]);
             }
             __syncthreads();
         }
-        V *C = static_cast<V *>(q.C) + b * q.m * q.n;
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -149,12 +205,19 @@ int jetgpu_contract_group(const jetgpu_group_task *tasks, int n_tasks, uint64_t 
     if (n_tasks == 0 || total_tiles == 0)
         return JETGPU_OK;
     JETGPU_REQUIRE(tasks != nullptr, "null task table");
-    const unsigned grid = GridFor(total_tiles, 8);
-    cudaStream_t st = AsStream(stream);
-    if (dtype == JETGPU_C64)
-        group_contract_kernel<float><<<grid, kGThreads, 0, st>>>(tasks, n_tasks, total_tiles);
-    else
-        group_contract_kernel<double><<<grid, kGThreads, 0, st>>>(tasks, n_tasks, total_tiles);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(GridFor(total_tiles, 8));
+    cfg.blockDim = dim3(kGThreads);
+    cfg.stream = AsStream(stream);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    JETGPU_CUDA_TRY(cudaLaunchKernelEx(&cfg,
+                                       dtype == JETGPU_C64 ? group_contract_kernel<float>
+                                                           : group_contract_kernel<double>,
+                                       tasks, n_tasks, total_tiles));
     return CheckLaunch("group_contract_kernel");
 }
 
