@@ -211,15 +211,25 @@ int GemmSplitPlanarBatched(const void *a_planes, int a_batched, const void *b_pl
                            cudaStream_t stream, int variant = -1,
                            const int *e_max_dev = nullptr, int group_m = 0,
                            int *out_emax = nullptr, unsigned int *tile_counter = nullptr,
-                           int algo = JETGPU_ALGO_4M);
+                           int algo = JETGPU_ALGO_4M, int splits = 1, void *partials = nullptr);
+
+// k ranges a split product of one m x n x k contraction is best cut into (1:
+// whole), and the bytes of partial sums they need: see gemm_tc.cu.
+int TcSplits(uint64_t m, uint64_t n, uint64_t k, SplitFormat fmt);
+
+// out[i] = sum over s < splits of part[s * len + i], added in FP64 in a fixed
+// order (complex64).
+int SumPartials(const void *part, void *out, uint64_t len, uint64_t splits, cudaStream_t stream);
 
 // Workspace bytes of a (batched) contraction in `precision` (JETGPU_PREC_TUNED:
-// the largest of its candidates' and AUTO's).
+// the largest of its candidates' and AUTO's). `single`: of jetgpu_contract,
+// whose product may cut k into ranges when it gets this much; `single` =
+// false is what every contraction accepts.
 size_t ContractWorkspace(uint64_t batch, int a_rank, const uint64_t *a_shape,
                          const int32_t *a_perm, int a_batched, int b_rank,
                          const uint64_t *b_shape, const int32_t *b_perm, int b_batched, uint64_t m,
                          uint64_t n, uint64_t k, int dtype, int precision,
-                         int algo = JETGPU_ALGO_4M);
+                         int algo = JETGPU_ALGO_4M, bool single = false);
 
 // Max-exponent hints of one contraction (device ints; each may be null):
 // `a` / `b` hold the operands' exponents when the kernels that wrote them
@@ -235,13 +245,16 @@ struct ExpHints {
 // A checked (batched) contraction in one form: precision FP32, TF32X3,
 // BF16X3, FP16X3 or AUTO; `variant` the tensor-core main loop (-1: the
 // jetgpu_set_tc_variant setting), `group_m` its tile order (0: the
-// jetgpu_set_tc_group_m setting).
+// jetgpu_set_tc_group_m setting). `single_ws`: bytes of the workspace of a
+// jetgpu_contract call, whose product may cut k into ranges with what is left
+// of it; 0 keeps the batched executors' order of additions.
 int ContractForm(uint64_t batch, const void *A, int a_rank, const uint64_t *a_shape,
                  const int32_t *a_perm, int a_batched, const void *B, int b_rank,
                  const uint64_t *b_shape, const int32_t *b_perm, int b_batched, void *C,
                  uint64_t m, uint64_t n, uint64_t k, int dtype, int precision, int variant,
                  int scale_a, int scale_b, void *workspace, cudaStream_t st, int group_m = 0,
-                 const ExpHints *hints = nullptr, int algo = JETGPU_ALGO_4M);
+                 const ExpHints *hints = nullptr, int algo = JETGPU_ALGO_4M,
+                 size_t single_ws = 0);
 
 // JETGPU_PREC_TUNED: the form the autotuner measured fastest for this
 // contraction's key, timing the candidates on first use (autotune.cu).

@@ -142,7 +142,8 @@ int SplitProduct(const SplitLayout &l, uint64_t batch, const void *A, int a_rank
                  const uint64_t *a_shape, const int32_t *a_perm, uint64_t ba, int a_mode,
                  const void *B, int b_rank, const uint64_t *b_shape, const int32_t *b_perm,
                  uint64_t bb, int b_mode, void *C, uint64_t m, uint64_t n, uint64_t k, int dtype,
-                 int scale_a, int scale_b, uint8_t *ws, cudaStream_t st, const ExpHints *hints)
+                 int scale_a, int scale_b, uint8_t *ws, cudaStream_t st, const ExpHints *hints,
+                 size_t single_ws)
 {
     int rc;
     uint8_t *pa = ws;
@@ -182,9 +183,15 @@ int SplitProduct(const SplitLayout &l, uint64_t batch, const void *A, int a_rank
                                  (b_mode == 2 ? bb : 1) * n, k, l.kp, bb * n * l.kp, scale_b,
                                  l.fmt, b_extra, st, e_dev ? e_dev + 1 : nullptr)))
         return rc;
+    // Partial sums of a cut k, behind everything above.
+    const size_t used = l.a_bytes(ba * m) + AlignUp(6 * bb * n * l.kp * l.word) + l.exp_bytes();
+    int splits = single_ws > used ? TcSplits(m, n, k, l.fmt) : 1;
+    if (splits > 1 && single_ws - used < (size_t)splits * m * n * sizeof(float2))
+        splits = 1;
     return GemmSplitPlanarBatched(pa, ba > 1, pb, bb > 1, C, batch, m, n, k, l.kp, out_scale,
                                   l.fmt, st, l.variant, e_dev, l.group_m,
-                                  hints ? hints->c : nullptr, tile_counter, l.algo);
+                                  hints ? hints->c : nullptr, tile_counter, l.algo, splits,
+                                  ws + used);
 }
 
 } // namespace
@@ -361,7 +368,7 @@ void FoldShape(int rank, const uint64_t *shape, const int32_t *perm, uint64_t ba
 size_t FormWorkspace(uint64_t batch, int a_rank, const uint64_t *a_shape, const int32_t *a_perm,
                      int a_batched, int b_rank, const uint64_t *b_shape, const int32_t *b_perm,
                      int b_batched, uint64_t m, uint64_t n, uint64_t k, int dtype, int precision,
-                     int algo = JETGPU_ALGO_4M)
+                     int algo = JETGPU_ALGO_4M, bool single = false)
 {
     if (batch <= 1 || (!a_batched && !b_batched)) {
         batch = 1;
@@ -381,7 +388,9 @@ size_t FormWorkspace(uint64_t batch, int a_rank, const uint64_t *a_shape, const 
     if (p.tc) {
         // Sized for six B planes whatever the main-loop variant.
         const SplitLayout l = LayoutFor(precision, k, (double)batch * m * n * k, -1, 0, algo);
-        return l.a_bytes(p.ba * m) + AlignUp(6 * p.bb * n * l.kp * l.word) + l.exp_bytes();
+        const int splits = single ? TcSplits(m, n, k, l.fmt) : 1;
+        return l.a_bytes(p.ba * m) + AlignUp(6 * p.bb * n * l.kp * l.word) + l.exp_bytes() +
+               (splits > 1 ? AlignUp((size_t)splits * m * n * sizeof(float2)) : 0);
     }
     if (k > 0 && SkinnyApplies(batch, a_rank, a_shape, a_perm, a_batched, b_rank, b_shape,
                                b_perm, b_batched, m, n, k))
@@ -402,11 +411,11 @@ size_t FormWorkspace(uint64_t batch, int a_rank, const uint64_t *a_shape, const 
 size_t ContractWorkspace(uint64_t batch, int a_rank, const uint64_t *a_shape,
                          const int32_t *a_perm, int a_batched, int b_rank,
                          const uint64_t *b_shape, const int32_t *b_perm, int b_batched, uint64_t m,
-                         uint64_t n, uint64_t k, int dtype, int precision, int algo)
+                         uint64_t n, uint64_t k, int dtype, int precision, int algo, bool single)
 {
     if (precision != JETGPU_PREC_TUNED)
         return FormWorkspace(batch, a_rank, a_shape, a_perm, a_batched, b_rank, b_shape, b_perm,
-                             b_batched, m, n, k, dtype, precision, algo);
+                             b_batched, m, n, k, dtype, precision, algo, single);
     // Any candidate of the tuner, and AUTO (untuned steps).
     size_t ws = 0;
     for (int prec : {JETGPU_PREC_FP32, JETGPU_PREC_AUTO, JETGPU_PREC_TF32X3, JETGPU_PREC_FP16X3}) {
@@ -424,7 +433,7 @@ int ContractForm(uint64_t batch, const void *A, int a_rank, const uint64_t *a_sh
                  const uint64_t *b_shape, const int32_t *b_perm, int b_batched, void *C,
                  uint64_t m, uint64_t n, uint64_t k, int dtype, int precision, int variant,
                  int scale_a, int scale_b, void *workspace, cudaStream_t st, int group_m,
-                 const ExpHints *hints, int algo)
+                 const ExpHints *hints, int algo, size_t single_ws)
 {
     if (batch <= 1 || (!a_batched && !b_batched)) {
         batch = 1;
@@ -449,7 +458,7 @@ int ContractForm(uint64_t batch, const void *A, int a_rank, const uint64_t *a_sh
                                       algo),
                             batch, A, a_rank, a_shape, a_perm, p.ba, p.ba > 1 ? a_batched : 0, B,
                             b_rank, b_shape, b_perm, p.bb, p.bb > 1 ? b_batched : 0, C, m, n, k,
-                            dtype, scale_a, scale_b, ws, st, hints);
+                            dtype, scale_a, scale_b, ws, st, hints, single_ws);
     if (k > 0 && SkinnyApplies(batch, a_rank, a_shape, a_perm, a_batched, b_rank, b_shape,
                                b_perm, b_batched, m, n, k))
         return SkinnyContract(batch, A, a_rank, a_shape, a_perm, a_batched, B, b_rank, b_shape,
@@ -540,7 +549,7 @@ int Contract(uint64_t batch, const void *A, int a_rank, const uint64_t *a_shape,
              const uint64_t *b_shape, const int32_t *b_perm, int b_batched, void *C, uint64_t m,
              uint64_t n, uint64_t k, int dtype, int precision, int algo, int scale_a, int scale_b,
              void *workspace, size_t workspace_bytes, cudaStream_t st,
-             const ExpHints *hints = nullptr)
+             const ExpHints *hints = nullptr, bool single = false)
 {
     bool empty = false;
     int rc = CheckContract(batch, A, a_rank, a_shape, a_perm, a_batched, B, b_rank, b_shape,
@@ -558,7 +567,7 @@ int Contract(uint64_t batch, const void *A, int a_rank, const uint64_t *a_shape,
                              st, hints);
     return ContractForm(batch, A, a_rank, a_shape, a_perm, a_batched, B, b_rank, b_shape, b_perm,
                         b_batched, C, m, n, k, dtype, precision, -1, scale_a, scale_b, workspace,
-                        st, 0, hints, algo);
+                        st, 0, hints, algo, single ? workspace_bytes : 0);
 }
 
 } // namespace
@@ -573,7 +582,7 @@ size_t jetgpu_contract_workspace_size(int a_rank, const uint64_t *a_shape,
                                       int precision)
 {
     return ContractWorkspace(1, a_rank, a_shape, a_perm, 0, b_rank, b_shape, b_perm, 0, m, n, k,
-                             dtype, precision);
+                             dtype, precision, JETGPU_ALGO_4M, true);
 }
 
 int jetgpu_contract(const void *A, int a_rank, const uint64_t *a_shape,
@@ -587,7 +596,7 @@ int jetgpu_contract(const void *A, int a_rank, const uint64_t *a_shape,
     ClearError();
     return Contract(1, A, a_rank, a_shape, a_perm, 0, B, b_rank, b_shape, b_perm, 0, C, m, n, k,
                     dtype, precision, algo, scale_a, scale_b, workspace, workspace_bytes,
-                    AsStream(stream));
+                    AsStream(stream), nullptr, true);
 }
 
 size_t jetgpu_contract_workspace_size_algo(int a_rank, const uint64_t *a_shape,
@@ -597,7 +606,7 @@ size_t jetgpu_contract_workspace_size_algo(int a_rank, const uint64_t *a_shape,
                                            int precision, int algo)
 {
     return ContractWorkspace(1, a_rank, a_shape, a_perm, 0, b_rank, b_shape, b_perm, 0, m, n, k,
-                             dtype, precision, algo);
+                             dtype, precision, algo, true);
 }
 
 size_t jetgpu_contract_batched_workspace_size(uint64_t batch, int a_rank, const uint64_t *a_shape,

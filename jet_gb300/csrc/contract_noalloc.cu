@@ -65,8 +65,9 @@ int jetgpu_contract_noalloc(const void *A, int a_rank, const uint64_t *a_shape,
                             int algo, int scale_a, int scale_b, void *stream)
 {
     jetgpu::ClearError();
-    const size_t need = jetgpu_contract_workspace_size(a_rank, a_shape, a_perm, b_rank, b_shape,
-                                                       b_perm, m, n, k, dtype, precision);
+    // What the contraction cannot do without; a cut of k takes room that is left.
+    const size_t need = jetgpu::ContractWorkspace(1, a_rank, a_shape, a_perm, 0, b_rank, b_shape,
+                                                  b_perm, 0, m, n, k, dtype, precision);
     if (need > jetgpu::kScratchBytes)
         return jetgpu::SetError(
             JETGPU_ERR_WORKSPACE,

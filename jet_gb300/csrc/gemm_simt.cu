@@ -892,6 +892,12 @@ int MultiplyPlainBatched(const void *A, const void *B, void *C, uint64_t batch, 
                                    stream);
 }
 
+int SumPartials(const void *part, void *out, uint64_t len, uint64_t splits, cudaStream_t stream)
+{
+    return ReducePartials<float>((const float2 *)part, (float2 *)out, (int64_t)len,
+                                 (int64_t)splits, stream);
+}
+
 size_t MultiplyPlainWorkspace(uint64_t m, uint64_t n, uint64_t k, int dtype)
 {
     return MultiplyPlainBatchedWorkspace(1, m, n, k, dtype);
