@@ -635,8 +635,27 @@ void BuildGather(const Simplified &s, uint64_t batch, GatherParams &p)
 // ---------------------------------------------------------------------------
 // Bit-permutation tiled kernel (power-of-2 tensors).
 // ---------------------------------------------------------------------------
-constexpr int kTileTables = 3; // 3 x 8 outer bits
+constexpr int kMaxOuter = 24; // bits that enumerate tiles
+// CTAs per SM of the grid (32 KB of shared memory each): six while the tensor
+// stays in L2, four from 2,048 tiles (64 MB) on, where more concurrent streams
+// cost DRAM pages: 2^27 complex64 with six / four CTAs: plain 371 / 328 us,
+// split stores 405 / 352. Registers for five: with six (40 registers) the
+// eight loads a warp should have in flight do not fit (371 us at four too).
+constexpr int kBitPerSm = 6;
+constexpr int kBitPerSmLarge = 4;
+constexpr int kBitResident = 5;
+constexpr uint64_t kBitLargeTiles = 2048;
 
+// Below this the gather kernel runs: its scattered reads hit L2, and it has no
+// barrier between its loads and stores. Measured in replayed graphs, random
+// orders, complex64: 2^13 2.2 us (tiles 2.9), 2^16 2.8 (3.2), 2^17 3.6 (3.3),
+// 2^18 5.7 (3.1); split stores 2^13 2.4 (3.8), 2^17 4.2 (4.0).
+constexpr uint64_t kBitMinBytes = 1ull << 20;
+
+// The plan travels as kernel parameters (constant memory), so it is small and
+// read uniformly: about 1.6 KB, where tables of tile bases (12 KB) and
+// per-lane entries cost a small permute a third of its time in constant-cache
+// misses. 2^18 elements 4.4 -> 3.1 us, 2^20 5.3 -> 4.1, 2^23 31.8 -> 26.7.
 struct BitParams {
     int n;       // bits of the linear index
     int u;       // tile bits
@@ -645,10 +664,13 @@ struct BitParams {
     uint64_t total_tiles;
     uint64_t in_hi[64];  // input offset of run h (h = L >> t)
     uint64_t out_hi[64]; // output offset of run h (h = M >> t)
-    uint32_t l_lo[64];   // tile-local input index of M & (2^t - 1)
     uint32_t l_hi[64];   // tile-local input index of (M >> t) << t
-    uint64_t tile_in[kTileTables][256];
-    uint64_t tile_out[kTileTables][256];
+    uint8_t lo_pos[8];   // tile-local input bit of output bit j < t
+    // Runs of tile bits that stay together: bits [src, src + width) of the
+    // tile number go to input bits from `in` and output bits from `out` on.
+    int n_seg;
+    uint8_t seg_src[kMaxOuter], seg_in[kMaxOuter], seg_out[kMaxOuter];
+    uint32_t seg_mask[kMaxOuter];
 };
 
 __device__ __forceinline__ uint32_t Swz(uint32_t h, int log_ve)
@@ -656,11 +678,33 @@ __device__ __forceinline__ uint32_t Swz(uint32_t h, int log_ve)
     return ((h ^ (h >> 5)) & 31u) << log_ve;
 }
 
-__device__ __forceinline__ uint64_t TileBase(const uint64_t (*tbl)[256],
-                                             uint64_t tt)
+// Segment s's share of the input and output offsets of tile tt. A warp's lane s
+// holds segment s, and the lanes' shares are ORed: a loop over the segments in
+// every thread made the split stores issue-bound (2^27 elements 4 % slower).
+struct BitSegment {
+    uint32_t src, in, out, mask;
+    __host__ __device__ BitSegment(const BitParams &p, int s)
+        : src(s < p.n_seg ? p.seg_src[s] : 0), in(s < p.n_seg ? p.seg_in[s] : 0),
+          out(s < p.n_seg ? p.seg_out[s] : 0), mask(s < p.n_seg ? p.seg_mask[s] : 0)
+    {
+    }
+    __host__ __device__ uint64_t In(uint32_t tt) const
+    {
+        return (uint64_t)((tt >> src) & mask) << in;
+    }
+    __host__ __device__ uint64_t Out(uint32_t tt) const
+    {
+        return (uint64_t)((tt >> src) & mask) << out;
+    }
+};
+
+// OR over the warp's lanes; the high words only for indices past 2^32.
+__device__ __forceinline__ uint64_t WarpOr(uint64_t v, bool wide)
 {
-    return tbl[0][tt & 255] + tbl[1][(tt >> 8) & 255] +
-           tbl[2][(tt >> 16) & 255];
+    uint64_t r = __reduce_or_sync(0xffffffffu, (uint32_t)v);
+    if (wide)
+        r |= (uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(v >> 32)) << 32;
+    return r;
 }
 
 // Store stage functor: plain element copy.
@@ -755,7 +799,7 @@ struct SplitStore {
 // E: element (uint2 = complex64, uint4 = complex128); LOG_VE: log2 of
 // elements per 16-byte vector.
 template <typename E, int LOG_VE, typename Store>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, kBitResident)
     bitperm_kernel(const __grid_constant__ BitParams p,
                    const E *__restrict__ in, Store store)
 {
@@ -771,17 +815,26 @@ __global__ void __launch_bounds__(kThreads)
 
     uint32_t llo[VE];
 #pragma unroll
-    for (int e = 0; e < VE; ++e)
-        llo[e] = p.l_lo[lane * VE + e];
+    for (int e = 0; e < VE; ++e) {
+        llo[e] = 0;
+#pragma unroll
+        for (int j = 0; j < 5 + LOG_VE; ++j)
+            llo[e] |= (((uint32_t)(lane * VE + e) >> j) & 1u) << p.lo_pos[j];
+    }
+    const BitSegment seg(p, lane);
+    // A warp's runs are consecutive: their table entries share cache lines.
+    const int per_warp = (runs + nwarps - 1) / nwarps;
+    const int h0 = warp * per_warp, h1 = min(runs, h0 + per_warp);
 
     for (uint64_t g = blockIdx.x; g < p.total_tiles; g += gridDim.x) {
         const uint64_t b = g >> p.n_outer;
-        const uint64_t tt = g & outer_mask;
-        const uint64_t in_base = (b << p.n) + TileBase(p.tile_in, tt);
-        const uint64_t out_base = (b << p.n) + TileBase(p.tile_out, tt);
+        const uint32_t tt = (uint32_t)(g & outer_mask);
+        const uint64_t in_base = (b << p.n) + WarpOr(seg.In(tt), p.n > 32);
+        const uint64_t out_base = (b << p.n) + WarpOr(seg.Out(tt), p.n > 32);
 
         // Load: run h covers tile-local input indices [h << t, (h+1) << t).
-        for (int h = warp; h < runs; h += nwarps) {
+#pragma unroll 8
+        for (int h = h0; h < h1; ++h) {
             const uint64_t off = in_base + p.in_hi[h] + (uint64_t)(lane * VE);
             uint4 v = __ldg(reinterpret_cast<const uint4 *>(in + off));
             const uint32_t L = ((uint32_t)h << t) | (uint32_t)(lane * VE);
@@ -790,7 +843,8 @@ __global__ void __launch_bounds__(kThreads)
         }
         __syncthreads();
         // Store: run h covers tile-local output indices [h << t, (h+1) << t).
-        for (int h = warp; h < runs; h += nwarps) {
+#pragma unroll 8
+        for (int h = h0; h < h1; ++h) {
             const uint32_t lhi = p.l_hi[h];
             E vals[VE];
 #pragma unroll
@@ -820,7 +874,9 @@ bool BuildBitParams(const Simplified &s, uint64_t batch, int log_ve,
     }
     const int t = 5 + log_ve;
     const int umax = log_ve == 1 ? 12 : 11; // 32 KB tile
-    if (n < umax || n - umax > 8 * kTileTables)
+    if (s.size * batch < (kBitMinBytes >> (log_ve == 1 ? 3 : 4)))
+        return false;
+    if (n < umax || n - umax > kMaxOuter)
         return false;
     // Input bit offsets of each input axis (axis r-1 is fastest).
     std::vector<int> in_off(r), out_off(r), out_axis_of_in(r);
@@ -892,27 +948,19 @@ bool BuildBitParams(const Simplified &s, uint64_t batch, int log_ve,
         p.out_hi[h] = vout;
         p.l_hi[h] = lh;
     }
-    for (int m = 0; m < (1 << t); ++m) {
-        uint32_t l = 0;
-        for (int j = 0; j < t; ++j)
-            if ((m >> j) & 1)
-                l |= 1u << pos_in_Us[src[Os[j]]];
-        p.l_lo[m] = l;
+    for (int j = 0; j < t; ++j)
+        p.lo_pos[j] = (uint8_t)pos_in_Us[src[Os[j]]];
+    for (size_t k = 0; k < Vs.size();) {
+        size_t e = k + 1;
+        while (e < Vs.size() && Vs[e] == Vs[e - 1] + 1 && dst[Vs[e]] == dst[Vs[e - 1]] + 1)
+            ++e;
+        p.seg_src[p.n_seg] = (uint8_t)k;
+        p.seg_in[p.n_seg] = (uint8_t)Vs[k];
+        p.seg_out[p.n_seg] = (uint8_t)dst[Vs[k]];
+        p.seg_mask[p.n_seg] = (uint32_t)((1ull << (e - k)) - 1);
+        ++p.n_seg;
+        k = e;
     }
-    const int nv = (int)Vs.size();
-    for (int k = 0; k < kTileTables; ++k)
-        for (int v = 0; v < 256; ++v) {
-            uint64_t ti = 0, to = 0;
-            for (int j = 0; j < 8; ++j) {
-                int bit = 8 * k + j;
-                if (bit < nv && ((v >> j) & 1)) {
-                    ti |= 1ull << Vs[bit];
-                    to |= 1ull << dst[Vs[bit]];
-                }
-            }
-            p.tile_in[k][v] = ti;
-            p.tile_out[k][v] = to;
-        }
     return true;
 }
 
@@ -928,7 +976,8 @@ int LaunchBitperm(const BitParams &p, const void *in, Store store,
             kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
         configured = true;
     }
-    unsigned grid = GridFor(p.total_tiles, 6);
+    unsigned grid = GridFor(p.total_tiles,
+                            p.total_tiles < kBitLargeTiles ? kBitPerSm : kBitPerSmLarge);
     kern<<<grid, kThreads, smem, stream>>>(p, reinterpret_cast<const E *>(in),
                                            store);
     return CheckLaunch("bitperm_kernel");
@@ -959,7 +1008,7 @@ int PermuteImpl(const void *in, void *out, uint64_t batch, int rank,
     }
     const bool aligned = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0);
     if (aligned) {
-        static thread_local BitParams bp; // ~14 KB: keep off the stack
+        static thread_local BitParams bp;
         if (dtype == JETGPU_C64 && BuildBitParams(s, batch, 1, bp))
             return LaunchBitperm<uint2, 1>(bp, in,
                                            PlainStore<uint2>{(uint2 *)out},
