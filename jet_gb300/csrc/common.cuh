@@ -127,6 +127,10 @@ int PermuteSplitTf32Batched(const void *in, float *planes, uint64_t batch, int r
 enum class SplitFormat { kTf32 = 0, kBf16 = 1, kFp16 = 2 };
 inline uint64_t SplitWordBytes(SplitFormat f) { return f == SplitFormat::kTf32 ? 4 : 2; }
 inline uint64_t SplitPitchAlign(SplitFormat f) { return f == SplitFormat::kTf32 ? 4 : 8; }
+// Paired planes: a row of the re (im) plane holds blocks of SplitPairWords hi
+// words followed by their lo words, 128 bytes a block, so that one TMA row
+// brings both. For columns in whole blocks.
+inline uint64_t SplitPairWords(SplitFormat f) { return f == SplitFormat::kTf32 ? 16 : 32; }
 
 // FP16 split: an operand whose largest magnitude has binary exponent e_max
 // (jetgpu_max_exponent; -1000 when all zero) is multiplied by 2^s before the
@@ -158,10 +162,13 @@ constexpr int kSplitNone = 0, kSplitNegIm = 1, kSplitSum = 2;
 // For FP16, `e_max_dev` points at the operand's max exponent on the device
 // and sets the scale (Fp16ScaleExp, one less with kSplitSum so the sums stay
 // in range); scale_exp is then ignored.
+// `paired`: two planes (re, im) of SplitPairWords blocks, `plane_stride` words
+// apart, row pitch `pitch` words; no extra pair.
 int PermuteSplitPlanes(const void *in, void *planes, uint64_t batch, int rank,
                        const uint64_t *shape, const int32_t *perm, uint64_t rows, uint64_t cols,
                        uint64_t pitch, uint64_t plane_stride, int scale_exp, SplitFormat fmt,
-                       int extra, cudaStream_t stream, const int *e_max_dev = nullptr);
+                       int extra, cudaStream_t stream, const int *e_max_dev = nullptr,
+                       bool paired = false);
 
 // Device max exponent of `size` complex elements into *e_dev (stream-ordered).
 int MaxExponent(const void *x, uint64_t size, int dtype, int *e_dev, cudaStream_t stream);
@@ -211,7 +218,8 @@ int GemmSplitPlanarBatched(const void *a_planes, int a_batched, const void *b_pl
                            cudaStream_t stream, int variant = -1,
                            const int *e_max_dev = nullptr, int group_m = 0,
                            int *out_emax = nullptr, unsigned int *tile_counter = nullptr,
-                           int algo = JETGPU_ALGO_4M, int splits = 1, void *partials = nullptr);
+                           int algo = JETGPU_ALGO_4M, int splits = 1, void *partials = nullptr,
+                           bool paired = false);
 
 // k ranges a split product of one m x n x k contraction is best cut into (1:
 // whole), and the bytes of partial sums they need: see gemm_tc.cu.

@@ -36,6 +36,7 @@ struct SplitLayout {
     int a_planes;     // 4, or 6 for 3M (re + im hi, lo)
     int b_planes;     // 4, or 6 for the N = 256 TF32 main loop and for 3M
     int group_m;      // tile order (0: the setting)
+    bool paired;      // two planes (re, im) of hi and lo blocks instead of four
     size_t a_bytes(uint64_t rows) const { return AlignUp(a_planes * rows * kp * word); }
     size_t b_bytes(uint64_t rows) const { return AlignUp(b_planes * rows * kp * word); }
     // After the planes: the operands' max exponents (two ints, FP16) and the
@@ -75,6 +76,9 @@ SplitLayout LayoutFor(int precision, uint64_t k, double work, int variant = -1,
     l.a_planes = algo == JETGPU_ALGO_3M ? 6 : 4;
     l.b_planes = (algo == JETGPU_ALGO_3M || l.variant == 1) ? 6 : 4;
     l.group_m = group_m;
+    // The default loops read paired planes where k is whole blocks; the same
+    // bytes either way.
+    l.paired = l.variant == 0 && algo == JETGPU_ALGO_4M && k % SplitPairWords(l.fmt) == 0;
     return l;
 }
 
@@ -174,24 +178,27 @@ int SplitProduct(const SplitLayout &l, uint64_t batch, const void *A, int a_rank
     // Mode 1: `ba` tensors back to back; mode 2: one tensor whose leading
     // permuted axes are the batch, i.e. ba * m rows of one split.
     const bool three_m = l.algo == JETGPU_ALGO_3M;
+    const uint64_t pair = l.paired ? 2 : 1; // a paired row holds hi and lo
     if ((rc = PermuteSplitPlanes(A, pa, a_mode == 1 ? ba : 1, a_rank, a_shape, a_perm,
-                                 (a_mode == 2 ? ba : 1) * m, k, l.kp, ba * m * l.kp, scale_a,
-                                 l.fmt, three_m ? kSplitSum : kSplitNone, st, e_dev)))
+                                 (a_mode == 2 ? ba : 1) * m, k, pair * l.kp, pair * ba * m * l.kp,
+                                 scale_a, l.fmt, three_m ? kSplitSum : kSplitNone, st, e_dev,
+                                 l.paired)))
         return rc;
     const int b_extra = three_m ? kSplitSum : (l.b_planes == 6 ? kSplitNegIm : kSplitNone);
     if ((rc = PermuteSplitPlanes(B, pb, b_mode == 1 ? bb : 1, b_rank, b_shape, bt.data(),
-                                 (b_mode == 2 ? bb : 1) * n, k, l.kp, bb * n * l.kp, scale_b,
-                                 l.fmt, b_extra, st, e_dev ? e_dev + 1 : nullptr)))
+                                 (b_mode == 2 ? bb : 1) * n, k, pair * l.kp, pair * bb * n * l.kp,
+                                 scale_b, l.fmt, b_extra, st, e_dev ? e_dev + 1 : nullptr,
+                                 l.paired)))
         return rc;
     // Partial sums of a cut k, behind everything above.
     const size_t used = l.a_bytes(ba * m) + AlignUp(6 * bb * n * l.kp * l.word) + l.exp_bytes();
     int splits = single_ws > used ? TcSplits(m, n, k, l.fmt) : 1;
     if (splits > 1 && single_ws - used < (size_t)splits * m * n * sizeof(float2))
         splits = 1;
-    return GemmSplitPlanarBatched(pa, ba > 1, pb, bb > 1, C, batch, m, n, k, l.kp, out_scale,
-                                  l.fmt, st, l.variant, e_dev, l.group_m,
+    return GemmSplitPlanarBatched(pa, ba > 1, pb, bb > 1, C, batch, m, n, k, pair * l.kp,
+                                  out_scale, l.fmt, st, l.variant, e_dev, l.group_m,
                                   hints ? hints->c : nullptr, tile_counter, l.algo, splits,
-                                  ws + used);
+                                  ws + used, l.paired);
 }
 
 } // namespace

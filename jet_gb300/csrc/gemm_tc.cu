@@ -21,20 +21,28 @@
 // tcgen05.commit; eight accumulator warps fold each finished K chunk into
 // FP32 registers (see the kernel comment) and write C.
 //
-// What bounds the product is the shared-memory port (128 bytes a clock): an
-// MMA of N = 128 reads 8 KB of operands in the 64 clocks it takes, the whole
-// port, and TMA writes the stages through the same port. N = 256 reads 12 KB
-// in 128 clocks. In the BF16 form the B planes lie in the stage as {Br_hi,
-// Bi_hi, Br_lo, Bi_lo}, so [Br; Bi] is one 256-row operand: Ar [Br; Bi] goes
-// into set 0 and Ai [Br; Bi] into set 1, all N = 256, 208 KB through the port
-// per 32 k instead of 256, and the fold adds (+, +) and (-, +), with half as
-// many terms per accumulator. Measured on M = 2^14, N = 2^12, K = 2^13, splits
-// included: 8.95 -> 8.20 ms at 4.5e-6 -> 4.4e-6 from FP64.
-// TF32 and FP16, the forms of whole networks, keep the N = 128 order: two sums
-// gave 6 % on a sliced 35-qubit amplitude but move its last bits, which
-// chunks, batches and resumed runs of one amplitude share; Ar [Br; Bi] as
-// N = 256 beside N = 128 for Ai (the same bits, 232 KB) measured no faster
-// there and 4 % slower on 2048 x 1024 x 1024.
+// What bounds the product. With its operands resident a stage's MMAs take
+// 1,536 clocks, as twelve of N = 128 (64 clocks each) or six of N = 256 (128)
+// per k step. The tensor core queues only a few of them, so whatever the issuing
+// thread does between the MMAs of two stages (barrier waits, ring positions) is
+// a gap, more easily behind N = 128. Clocks per stage of one CTA on an idle GPU:
+// FP16 and TF32 2,460 -> 2,070 by counting ring positions instead of dividing
+// and by waiting for the next stage behind the current one's first MMAs; BF16
+// 1,990 -> 1,750. Past that, large products draw the GPU's 1.4 kW and clock down
+// to 1.7 GHz.
+//  * BF16: the B planes lie in the stage so that [Br; Bi] is one 256-row
+//    operand: Ar [Br; Bi] goes into set 0 and Ai [Br; Bi] into set 1, all N =
+//    256, and the fold adds (+, +) and (-, +), with half as many terms per
+//    accumulator. M = 2^14, N = 2^12, K = 2^13, splits included: 8.95 -> 8.20 ms
+//    at 4.5e-6 -> 4.4e-6 from FP64.
+//  * TF32 and FP16, the forms of whole networks, keep every accumulator's order
+//    of terms, and so their bits, which chunks, batches and resumed runs of one
+//    amplitude share: Ar [Br; Bi] as N = 256 (paired planes), Ai as N = 128. Two
+//    sums gave a few per cent on a sliced amplitude but move its last bits.
+//  * Contractions whose k is whole blocks write paired planes: 128-byte rows of
+//    hi and lo words, half the rows for TMA, which moves one a clock. 35-qubit
+//    sliced amplitude 8.72 -> 8.54 ms, 2^14 x 2^12 x 2^13 8.23 -> 7.94 ms (with
+//    the shorter gaps 7.88 and 7.69).
 // The 3M ("Gauss") form uses three real products instead of four:
 //   P1 = Ar Br,  P2 = Ai Bi,  P3 = (Ar + Ai)(Br + Bi),
 //   Cr = P1 - P2,  Ci = P3 - P1 - P2,
@@ -87,6 +95,10 @@ constexpr int kTileRing = 4;                  // tile indices in flight between 
 //  8, 9 BF16 / FP16 wide: variant 1's N = 256 main loop on 16-bit planes
 //                 (two stages of 4 A + 6 B boxes of 32 k; the B triples of
 //                 variant 1 with the negated imaginary planes).
+//  10, 11, 12     TF32 / BF16 / FP16 paired: variants 0, 2, 4 on paired planes
+//                 (a contraction's own splits): 3 stages of four boxes (Ar, Ai,
+//                 Br, Bi) of 128 rows x 128 bytes, a row holding 64 bytes of hi
+//                 words and their lo words, 128-byte swizzle.
 //  5, 6, 7 3M:    TF32 / BF16 / FP16 planes, 64-byte rows, 2 stages of six A
 //                 plane boxes (re, im, re + im; hi, lo) and six B boxes;
 //                 9 MMAs of N = 128 per k step, each product into its own
@@ -134,9 +146,26 @@ template <> struct TcCfg<7> {
     static constexpr bool Wide = false, ThreeM = true;
     static constexpr int Fmt = kFmtFp16, Stages = 2, Tiles = 12, RowBytes = 64;
 };
+template <> struct TcCfg<10> {
+    static constexpr bool Wide = false, ThreeM = false;
+    static constexpr int Fmt = kFmtTf32, Stages = 3, Tiles = 4, RowBytes = 128;
+};
+template <> struct TcCfg<11> {
+    static constexpr bool Wide = false, ThreeM = false;
+    static constexpr int Fmt = kFmtBf16, Stages = 3, Tiles = 4, RowBytes = 128;
+};
+template <> struct TcCfg<12> {
+    static constexpr bool Wide = false, ThreeM = false;
+    static constexpr int Fmt = kFmtFp16, Stages = 3, Tiles = 4, RowBytes = 128;
+};
+// Paired planes: a 128-byte row is 64 bytes of hi words, then their lo words.
+template <int V> constexpr bool Paired() { return TcCfg<V>::RowBytes == 128; }
 template <int V> constexpr int TileBytes() { return kBM * TcCfg<V>::RowBytes; }
 template <int V> constexpr int ElemBytes() { return TcCfg<V>::Fmt == kFmtTf32 ? 4 : 2; }
-template <int V> constexpr int BlockK() { return TcCfg<V>::RowBytes / ElemBytes<V>(); }
+template <int V> constexpr int BlockK()
+{
+    return TcCfg<V>::RowBytes / ElemBytes<V>() / (Paired<V>() ? 2 : 1);
+}
 template <int V> constexpr int StageBytes() { return TcCfg<V>::Tiles * TileBytes<V>(); }
 
 // Default K depth accumulated in TMEM per chunk. TF32: 16, one fold per
@@ -253,13 +282,13 @@ __device__ __forceinline__ void TmaLoad4d(uint32_t dst, const CUtensorMap *map,
 // 8-row groups 8 * kRow bytes apart.
 template <int kRow> __device__ __forceinline__ uint64_t SmemDesc(uint32_t addr)
 {
-    static_assert(kRow == 64 || kRow == 32, "64- or 32-byte rows");
+    static_assert(kRow == 128 || kRow == 64 || kRow == 32, "128-, 64- or 32-byte rows");
     uint64_t d = 0;
     d |= (uint64_t)((addr & 0x3FFFFu) >> 4);                 // start address
     d |= (uint64_t)1 << 16;                                  // leading byte offset (unused)
     d |= (uint64_t)((8 * kRow) >> 4) << 32;                  // stride byte offset
     d |= (uint64_t)1 << 46;                                  // descriptor version
-    d |= (uint64_t)(kRow == 64 ? 4 : 6) << 61;               // swizzle mode
+    d |= (uint64_t)(kRow == 128 ? 2 : kRow == 64 ? 4 : 6) << 61; // swizzle mode
     return d;
 }
 
@@ -395,7 +424,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     using Cfg = TcCfg<V>;
     constexpr bool kWide = Cfg::Wide;
     constexpr bool kThreeM = Cfg::ThreeM;
-    constexpr int kAPlanes = kThreeM ? 6 : 4;
+    constexpr bool kPaired = Paired<V>();
+    constexpr int kAPlanes = kThreeM ? 6 : kPaired ? 2 : 4;
+    // Bytes of K per row and stage, in MMAs of 32 bytes each.
+    constexpr int kKSteps = Cfg::RowBytes / 32 / (kPaired ? 2 : 1);
     constexpr int kFmt = Cfg::Fmt;
     constexpr bool kHalf = kFmt != kFmtTf32;
     constexpr bool kTwoSums = kFmt == kFmtBf16 && !kWide && !kThreeM;
@@ -486,6 +518,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (lane == 0) {
             // Tile scheduler and TMA producer.
             bool ok = true;
+            int s = 0; // stage-ring position and parity, running on across tiles
+            uint32_t phase = 0;
             for (int i = 0; ok; ++i) {
             const int r = i % kTileRing;
             if (!MbarWait(SmemAddr(&tile_empty[r]), ((uint32_t)(i / kTileRing) & 1u) ^ 1u))
@@ -502,9 +536,6 @@ __global__ void __launch_bounds__(kThreads, 1)
             int bz, m0, n0;
             tile_at(t, bz, m0, n0);
             for (int kt = 0; kt < ktiles; ++kt) {
-                const long long g = (long long)i * ktiles + kt; // stage-ring position
-                const int s = (int)(g % kStages);
-                const uint32_t phase = (uint32_t)(g / kStages) & 1u;
                 if (!MbarWait(SmemAddr(&empty_bar[s]), phase ^ 1u)) {
                     ok = false;
                     break;
@@ -512,7 +543,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const uint32_t fb = SmemAddr(&full_bar[s]);
                 MbarArriveExpectTx(fb, kStageBytes);
                 const uint32_t base = SmemAddr(smem + s * kStageBytes);
-                const int k0 = ((total_ktiles > 0 ? bz * ktiles : 0) + kt) * kBK;
+                const int k0 = ((total_ktiles > 0 ? bz * ktiles : 0) + kt) * kBK *
+                               (kPaired ? 2 : 1);
 #pragma unroll
                 for (int p = 0; p < kAPlanes; ++p) {
                     if (a_batched)
@@ -530,13 +562,17 @@ __global__ void __launch_bounds__(kThreads, 1)
                 for (int t = 0; t < kBTiles; ++t) {
                     const int plane = kWide      ? (t == 0 ? 4 : t == 1 ? 0 : t == 2 ? 2
                                                     : t == 3 ? 5 : t == 4 ? 1 : 3)
-                                      : kTwoSums ? (t & 1) * 2 + (t >> 1)
-                                                 : t;
+                                      : kTwoSums && !kPaired ? (t & 1) * 2 + (t >> 1)
+                                                             : t;
                     if (b_batched)
                         TmaLoad4d(base + (kAPlanes + t) * kTileBytes, &tmB, k0, n0, bz, plane,
                                   fb);
                     else
                         TmaLoad3d(base + (kAPlanes + t) * kTileBytes, &tmB, k0, n0, plane, fb);
+                }
+                if (++s == kStages) {
+                    s = 0;
+                    phase ^= 1u;
                 }
             }
             }
@@ -549,6 +585,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             constexpr uint32_t kIdesc = InstrDesc(kBM, kBN, false, kFmt);
             constexpr uint32_t kIdescNeg = InstrDesc(kBM, kBN, true, kFmt);
             bool ok = true;
+            // Stage-ring position and parity, and folds handed over so far,
+            // running on across tiles: counted, not divided, because the
+            // tensor core queues only a few MMAs, so every clock between the
+            // MMAs of two stages is a gap (64-bit divisions here took 260 of
+            // 2,460 clocks a stage).
+            int s = 0;
+            uint32_t phase = 0, gc = 0;
             for (int i = 0; ok; ++i) {
             const int r = i % kTileRing;
             if (!MbarWait(SmemAddr(&tile_full[r]), (uint32_t)(i / kTileRing) & 1u))
@@ -561,9 +604,6 @@ __global__ void __launch_bounds__(kThreads, 1)
                 break;
             if constexpr (kThreeM) {
             for (int kt = 0; kt < ktiles && ok; ++kt) {
-                const long long g = (long long)i * ktiles + kt;
-                const int s = (int)(g % kStages);
-                const uint32_t phase = (uint32_t)(g / kStages) & 1u;
                 if (!MbarWait(SmemAddr(&full_bar[s]), phase)) {
                     ok = false;
                     break;
@@ -574,9 +614,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                 for (int p = 0; p < 3; ++p) {
                     // Product p of stage g into slot q mod 4, free once the
                     // product four back has been folded.
-                    const long long q = 3 * g + p;
-                    const int slot = (int)(q & 3);
-                    if (!MbarWait(SmemAddr(&acc_empty[slot]), ((uint32_t)(q >> 2) & 1u) ^ 1u)) {
+                    const int slot = (int)(gc & 3u);
+                    if (!MbarWait(SmemAddr(&acc_empty[slot]), ((gc >> 2) & 1u) ^ 1u)) {
                         ok = false;
                         break;
                     }
@@ -598,21 +637,23 @@ __global__ void __launch_bounds__(kThreads, 1)
                         Mma<kHalf>(d, al, bh, kIdesc, 1u);
                     }
                     MmaCommit(SmemAddr(&acc_full[slot]));
+                    ++gc;
                 }
                 MmaCommit(SmemAddr(&empty_bar[s]));
+                if (++s == kStages) {
+                    s = 0;
+                    phase ^= 1u;
+                }
             }
             }
             else if constexpr (kTwoSums) {
             constexpr uint32_t kIdesc2 = InstrDesc(kBM, 2 * kBN, false, kFmt);
             int in_chunk = 0;
             for (int kt = 0; kt < ktiles && ok; ++kt) {
-                const long long gc = (long long)i * nchunks + kt / chunk_stages;
                 const bool chunk_start = in_chunk == 0;
                 const bool chunk_end = in_chunk == chunk_stages - 1 || kt == ktiles - 1;
                 in_chunk = chunk_end ? 0 : in_chunk + 1;
-                const long long g = (long long)i * ktiles + kt;
-                const int s = (int)(g % kStages);
-                if (!MbarWait(SmemAddr(&full_bar[s]), (uint32_t)(g / kStages) & 1u)) {
+                if (!MbarWait(SmemAddr(&full_bar[s]), phase)) {
                     ok = false;
                     break;
                 }
@@ -621,7 +662,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) { // set 0: Ar [Br; Bi], set 1: Ai [Br; Bi]
                     if (chunk_start) {
-                        if (!MbarWait(SmemAddr(&acc_empty[h]), ((uint32_t)gc & 1u) ^ 1u)) {
+                        if (!MbarWait(SmemAddr(&acc_empty[h]), (gc & 1u) ^ 1u)) {
                             ok = false;
                             break;
                         }
@@ -629,14 +670,17 @@ __global__ void __launch_bounds__(kThreads, 1)
                     }
                     const uint32_t d = tmem + h * 2 * kBN;
 #pragma unroll
-                    for (int kk = 0; kk < kRowBytes / 32; ++kk) {
+                    for (int kk = 0; kk < kKSteps; ++kk) {
                         const uint32_t koff = kk * 32; // 32 bytes of K per MMA
-                        const uint64_t ah =
-                            SmemDesc<kRowBytes>(base + (2 * h) * kTileBytes + koff);
-                        const uint64_t al =
-                            SmemDesc<kRowBytes>(base + (2 * h + 1) * kTileBytes + koff);
-                        const uint64_t bh = SmemDesc<kRowBytes>(base + 4 * kTileBytes + koff);
-                        const uint64_t bl = SmemDesc<kRowBytes>(base + 6 * kTileBytes + koff);
+                        const uint64_t ah = SmemDesc<kRowBytes>(
+                            base + (kPaired ? h : 2 * h) * kTileBytes + koff);
+                        const uint64_t al = SmemDesc<kRowBytes>(
+                            base + (kPaired ? h * kTileBytes + 64 : (2 * h + 1) * kTileBytes) +
+                            koff);
+                        const uint64_t bh =
+                            SmemDesc<kRowBytes>(base + kAPlanes * kTileBytes + koff);
+                        const uint64_t bl = SmemDesc<kRowBytes>(
+                            base + (kPaired ? kAPlanes * kTileBytes + 64 : 6 * kTileBytes) + koff);
                         Mma<kHalf>(d, ah, bh, kIdesc2, (chunk_start && kk == 0) ? 0u : 1u);
                         Mma<kHalf>(d, ah, bl, kIdesc2, 1u);
                         Mma<kHalf>(d, al, bh, kIdesc2, 1u);
@@ -646,29 +690,41 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
                 if (ok)
                     MmaCommit(SmemAddr(&empty_bar[s]));
+                gc += chunk_end ? 1u : 0u;
+                if (++s == kStages) {
+                    s = 0;
+                    phase ^= 1u;
+                }
             }
             }
-            else
+            else {
+            int in_chunk = 0;
+            bool ready = false; // this stage's waits are done
             for (int kt = 0; kt < ktiles && ok; ++kt) {
-                const int chunk = kt / chunk_stages;
                 // Accumulator set: chunks alternate across tiles too.
-                const long long gc = (long long)i * nchunks + chunk;
-                const int buf = (int)(gc & 1);
-                const int in_chunk = kt - chunk * chunk_stages;
+                const int buf = (int)(gc & 1u);
                 const bool chunk_start = in_chunk == 0;
                 const bool chunk_end = in_chunk == chunk_stages - 1 || kt == ktiles - 1;
-                if (chunk_start &&
-                    !MbarWait(SmemAddr(&acc_empty[buf]), ((uint32_t)(gc >> 1) & 1u) ^ 1u)) {
-                    ok = false;
+                in_chunk = chunk_end ? 0 : in_chunk + 1;
+                if (!ready)
+                    ok = (!chunk_start ||
+                          MbarWait(SmemAddr(&acc_empty[buf]), ((gc >> 1) & 1u) ^ 1u)) &&
+                         MbarWait(SmemAddr(&full_bar[s]), phase);
+                if (!ok)
                     break;
-                }
-                const long long g = (long long)i * ktiles + kt;
-                const int s = (int)(g % kStages);
-                const uint32_t phase = (uint32_t)(g / kStages) & 1u;
-                if (!MbarWait(SmemAddr(&full_bar[s]), phase)) {
-                    ok = false;
-                    break;
-                }
+                // The next stage's waits, behind this stage's first MMAs: the
+                // tensor core works through those meanwhile (2,070 clocks a
+                // stage; 2,190 without). Not in the wide loop, whose ring of two
+                // stages has the next one still loading, nor between the N = 256
+                // MMAs of the BF16 loop (1,750 clocks without, 1,830 with).
+                const auto prepare_next = [&] {
+                    ready = kt + 1 < ktiles;
+                    const int sn = s + 1 == kStages ? 0 : s + 1;
+                    if (ready)
+                        ok = (!chunk_end || MbarWait(SmemAddr(&acc_empty[buf ^ 1]),
+                                                     (((gc + 1u) >> 1) & 1u) ^ 1u)) &&
+                             MbarWait(SmemAddr(&full_bar[sn]), phase ^ (sn == 0));
+                };
                 FenceAfterSync();
                 const uint32_t d_re = tmem + buf * 2 * kBN;
                 const uint32_t d_im = d_re + kBN;
@@ -700,37 +756,58 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
                 else
 #pragma unroll
-                for (int kk = 0; kk < kRowBytes / 32; ++kk) {
+                for (int kk = 0; kk < kKSteps; ++kk) {
                     const uint32_t koff = kk * 32; // 32 bytes of K per MMA
-                    const uint64_t arh = SmemDesc<kRowBytes>(base + 0 * kTileBytes + koff);
-                    const uint64_t arl = SmemDesc<kRowBytes>(base + 1 * kTileBytes + koff);
-                    const uint64_t aih = SmemDesc<kRowBytes>(base + 2 * kTileBytes + koff);
-                    const uint64_t ail = SmemDesc<kRowBytes>(base + 3 * kTileBytes + koff);
-                    const uint64_t brh = SmemDesc<kRowBytes>(base + 4 * kTileBytes + koff);
-                    const uint64_t brl = SmemDesc<kRowBytes>(base + 5 * kTileBytes + koff);
-                    const uint64_t bih = SmemDesc<kRowBytes>(base + 6 * kTileBytes + koff);
-                    const uint64_t bil = SmemDesc<kRowBytes>(base + 7 * kTileBytes + koff);
+                    // Operand q (0 Ar, 1 Ai, 2 Br, 3 Bi), hi or lo piece.
+                    const auto operand = [&](int q, int lo) {
+                        return SmemDesc<kRowBytes>(
+                            base + (kPaired ? q * kTileBytes + 64 * lo : (2 * q + lo) * kTileBytes) +
+                            koff);
+                    };
+                    const uint64_t arh = operand(0, 0), arl = operand(0, 1);
+                    const uint64_t aih = operand(1, 0), ail = operand(1, 1);
+                    const uint64_t brh = operand(2, 0), brl = operand(2, 1);
+                    const uint64_t bih = operand(3, 0), bil = operand(3, 1);
                     const uint32_t acc = (chunk_start && kk == 0) ? 0u : 1u;
-                    // Cr += Ar Br
-                    Mma<kHalf>(d_re, arh, brh, kIdesc, acc);
-                    Mma<kHalf>(d_re, arh, brl, kIdesc, 1u);
-                    Mma<kHalf>(d_re, arl, brh, kIdesc, 1u);
+                    if constexpr (kPaired) {
+                        // (Cr | Ci) += Ar [Br; Bi]
+                        constexpr uint32_t kIdesc2 = InstrDesc(kBM, 2 * kBN, false, kFmt);
+                        Mma<kHalf>(d_re, arh, brh, kIdesc2, acc);
+                        Mma<kHalf>(d_re, arh, brl, kIdesc2, 1u);
+                        Mma<kHalf>(d_re, arl, brh, kIdesc2, 1u);
+                    }
+                    else {
+                        // Cr += Ar Br
+                        Mma<kHalf>(d_re, arh, brh, kIdesc, acc);
+                        Mma<kHalf>(d_re, arh, brl, kIdesc, 1u);
+                        Mma<kHalf>(d_re, arl, brh, kIdesc, 1u);
+                    }
                     // Cr -= Ai Bi
                     Mma<kHalf>(d_re, aih, bih, kIdescNeg, 1u);
                     Mma<kHalf>(d_re, aih, bil, kIdescNeg, 1u);
                     Mma<kHalf>(d_re, ail, bih, kIdescNeg, 1u);
-                    // Ci += Ar Bi
-                    Mma<kHalf>(d_im, arh, bih, kIdesc, acc);
-                    Mma<kHalf>(d_im, arh, bil, kIdesc, 1u);
-                    Mma<kHalf>(d_im, arl, bih, kIdesc, 1u);
+                    if constexpr (!kPaired) {
+                        // Ci += Ar Bi
+                        Mma<kHalf>(d_im, arh, bih, kIdesc, acc);
+                        Mma<kHalf>(d_im, arh, bil, kIdesc, 1u);
+                        Mma<kHalf>(d_im, arl, bih, kIdesc, 1u);
+                    }
                     // Ci += Ai Br
                     Mma<kHalf>(d_im, aih, brh, kIdesc, 1u);
                     Mma<kHalf>(d_im, aih, brl, kIdesc, 1u);
                     Mma<kHalf>(d_im, ail, brh, kIdesc, 1u);
+                    if (kk == 0)
+                        prepare_next();
                 }
                 MmaCommit(SmemAddr(&empty_bar[s]));
                 if (chunk_end)
                     MmaCommit(SmemAddr(&acc_full[buf]));
+                gc += chunk_end ? 1u : 0u;
+                if (++s == kStages) {
+                    s = 0;
+                    phase ^= 1u;
+                }
+            }
             }
             }
         }
@@ -998,8 +1075,15 @@ int GetEncoder()
     return JETGPU_OK;
 }
 
+CUtensorMapSwizzle Swizzle(int row_bytes)
+{
+    return row_bytes == 128  ? CU_TENSOR_MAP_SWIZZLE_128B
+           : row_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                             : CU_TENSOR_MAP_SWIZZLE_32B;
+}
+
 // 3-D map over planes: (k, row, plane), box (row_bytes of k) x 128 x 1,
-// swizzled over row_bytes (64 or 32).
+// swizzled over row_bytes (128, 64 or 32).
 int EncodePlanes(CUtensorMap *map, const void *base, uint64_t rows, uint64_t k,
                  uint64_t kpitch, bool half, int planes, int row_bytes)
 {
@@ -1012,8 +1096,8 @@ int EncodePlanes(CUtensorMap *map, const void *base, uint64_t rows, uint64_t k,
                           half ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
                           3, const_cast<void *>(base), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          row_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                          Swizzle(row_bytes), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
         return SetError(JETGPU_ERR_CUDA,
                         "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
@@ -1034,8 +1118,8 @@ int EncodePlanesBatched(CUtensorMap *map, const void *base, uint64_t rows, uint6
                           half ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
                           4, const_cast<void *>(base), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          row_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                          Swizzle(row_bytes), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
         return SetError(JETGPU_ERR_CUDA,
                         "cuTensorMapEncodeTiled (4-D) failed: " + std::to_string((int)r));
@@ -1162,7 +1246,7 @@ int LaunchSplitProduct(const void *a_planes, int a_batched, const void *b_planes
                        void *C, uint64_t batch, uint64_t m, uint64_t n, uint64_t k,
                        uint64_t kpitch, float out_scale, SplitFormat fmt, cudaStream_t stream,
                        int variant, const int *e_max_dev, int group_m, int *out_emax,
-                       unsigned int *tile_counter, int algo, int splits)
+                       unsigned int *tile_counter, int algo, int splits, bool paired)
 {
     JETGPU_REQUIRE(algo == JETGPU_ALGO_4M || algo == JETGPU_ALGO_3M, "bad algorithm");
     const bool three_m = algo == JETGPU_ALGO_3M;
@@ -1178,7 +1262,9 @@ int LaunchSplitProduct(const void *a_planes, int a_batched, const void *b_planes
     JETGPU_REQUIRE(m > 0 && n > 0 && k > 0, "empty product");
     JETGPU_REQUIRE(m < (1ull << 31) && n < (1ull << 31) && k < (1ull << 31),
                    "dimension too large");
-    JETGPU_REQUIRE(kpitch >= k && kpitch % SplitPitchAlign(fmt) == 0, "bad k pitch");
+    JETGPU_REQUIRE(kpitch >= (paired ? 2 : 1) * k && kpitch % SplitPitchAlign(fmt) == 0,
+                   "bad k pitch");
+    JETGPU_REQUIRE(!paired || k % SplitPairWords(fmt) == 0, "paired planes need whole blocks");
     JETGPU_REQUIRE(((uintptr_t)a_planes % 16) == 0 && ((uintptr_t)b_planes % 16) == 0,
                    "planes must be 16-byte aligned");
     JETGPU_REQUIRE(((n + kBN - 1) / kBN) * ((m + kBM - 1) / kBM) <= 0x7fffffffull,
@@ -1192,19 +1278,35 @@ int LaunchSplitProduct(const void *a_planes, int a_batched, const void *b_planes
         variant = TcVariant();
     const bool wide = variant == 1 && !three_m;
     const bool deep = bf16 && variant == 2 && !three_m;
-    const int row_bytes = deep ? TcCfg<3>::RowBytes : TcCfg<0>::RowBytes;
-    const int aplanes = three_m ? 6 : 4;
+    JETGPU_REQUIRE(!paired || (variant == 0 && !three_m), "paired planes have their own loops");
+    const int row_bytes = paired ? TcCfg<10>::RowBytes
+                          : deep ? TcCfg<3>::RowBytes
+                                 : TcCfg<0>::RowBytes;
+    const int aplanes = three_m ? 6 : paired ? 2 : 4;
+    // Words of a row: hi and lo in a paired row; else k, past which a box reads
+    // zeros.
+    const uint64_t kw = paired ? 2 * k : k;
     CUtensorMap ta, tb;
     if ((rc = a_batched
-                  ? EncodePlanesBatched(&ta, a_planes, m, k, kpitch, batch, half, aplanes,
+                  ? EncodePlanesBatched(&ta, a_planes, m, kw, kpitch, batch, half, aplanes,
                                         row_bytes)
-                  : EncodePlanes(&ta, a_planes, m, k, kpitch, half, aplanes, row_bytes)))
+                  : EncodePlanes(&ta, a_planes, m, kw, kpitch, half, aplanes, row_bytes)))
         return rc;
-    const int bplanes = (wide || three_m) ? 6 : 4;
-    if ((rc = b_batched
-                  ? EncodePlanesBatched(&tb, b_planes, n, k, kpitch, batch, half, bplanes, row_bytes)
-                  : EncodePlanes(&tb, b_planes, n, k, kpitch, half, bplanes, row_bytes)))
+    const int bplanes = (wide || three_m) ? 6 : paired ? 2 : 4;
+    if ((rc = b_batched ? EncodePlanesBatched(&tb, b_planes, n, kw, kpitch, batch, half, bplanes,
+                                              row_bytes)
+                        : EncodePlanes(&tb, b_planes, n, kw, kpitch, half, bplanes, row_bytes)))
         return rc;
+    if (paired) {
+        if (fp16)
+            return LaunchTc<12>(ta, tb, C, batch, m, n, k, out_scale, a_batched, b_batched,
+                                stream, e_max_dev, group_m, out_emax, tile_counter, splits);
+        if (bf16)
+            return LaunchTc<11>(ta, tb, C, batch, m, n, k, out_scale, a_batched, b_batched,
+                                stream, nullptr, group_m, out_emax, tile_counter, splits);
+        return LaunchTc<10>(ta, tb, C, batch, m, n, k, out_scale, a_batched, b_batched, stream,
+                            nullptr, group_m, out_emax, tile_counter, splits);
+    }
     if (three_m) {
         if (fp16)
             return LaunchTc<7>(ta, tb, C, batch, m, n, k, out_scale, a_batched, b_batched,
@@ -1268,19 +1370,19 @@ int GemmSplitPlanarBatched(const void *a_planes, int a_batched, const void *b_pl
                            uint64_t k, uint64_t kpitch, float out_scale, SplitFormat fmt,
                            cudaStream_t stream, int variant, const int *e_max_dev, int group_m,
                            int *out_emax, unsigned int *tile_counter, int algo, int splits,
-                           void *partials)
+                           void *partials, bool paired)
 {
     if (splits > 1) { // the ranges' sums beside each other, then their sum
         JETGPU_REQUIRE(batch == 1 && partials != nullptr && out_emax == nullptr,
                        "only one product is cut into k ranges");
         const int rc = LaunchSplitProduct(a_planes, 0, b_planes, 0, partials, 1, m, n, k, kpitch,
                                           out_scale, fmt, stream, variant, e_max_dev, group_m,
-                                          nullptr, tile_counter, algo, splits);
+                                          nullptr, tile_counter, algo, splits, paired);
         return rc ? rc : SumPartials(partials, C, m * n, (uint64_t)splits, stream);
     }
     return LaunchSplitProduct(a_planes, a_batched, b_planes, b_batched, C, batch, m, n, k, kpitch,
                               out_scale, fmt, stream, variant, e_max_dev, group_m, out_emax,
-                              tile_counter, algo, 1);
+                              tile_counter, algo, 1, paired);
 }
 int TcVariant() { return g_tc_variant.load(std::memory_order_relaxed); }
 bool TcWide() { return TcVariant() == 1; }

@@ -220,6 +220,8 @@ struct SplitOut {
     int fp16;              // 16-bit FP16 words of the operand scaled by its FP16 scale
     const int *e_max_dev;  // FP16: the operand's max exponent (sets the scale)
     int cols_log2;         // log2(cols) when cols is a power of 2 (bit-permutation path)
+    uint64_t lo_stride, im_stride; // words from a hi word to its lo word, and from re to im
+    int pair_log2;         // paired planes: log2 of SplitPairWords; 0: planar
     uint32_t cols_magic, cols_shift; // division by cols (DivMagic)
     int narrow;            // fewer than 2^32 elements: 32-bit rows and columns
 };
@@ -242,6 +244,15 @@ __device__ __forceinline__ void Split16x2(const SplitOut &so, float x0, float x1
         SplitBf16x2(x0, x1, hi, lo);
 }
 
+// Word offset of (row, col) in the re_hi plane.
+__device__ __forceinline__ uint64_t SplitOffset(const SplitOut &so, uint64_t row, uint64_t col)
+{
+    if (so.pair_log2)
+        return row * so.pitch + ((col >> so.pair_log2) << (so.pair_log2 + 1)) +
+               (col & ((1u << so.pair_log2) - 1));
+    return row * so.pitch + col;
+}
+
 // Writes element o of the split view; sc is SplitScale(so), which a kernel
 // reads once (after each store it would be read again: the planes might alias
 // it). A 64-bit division per element, and that read, made the qutrit split
@@ -258,16 +269,16 @@ __device__ __forceinline__ void WriteSplit(const SplitOut &so, uint64_t o, float
         row = o / so.cols;
         col = o - row * so.cols;
     }
-    const uint64_t off = row * so.pitch + col;
+    const uint64_t off = SplitOffset(so, row, col);
     float re = v.x * sc, im = v.y * sc;
     if (so.bf16 || so.fp16) {
         uint16_t *pl = static_cast<uint16_t *>(so.planes);
         uint32_t h, l; // (re, im) packed
         Split16x2(so, re, im, h, l);
         pl[off] = (uint16_t)(h & 0xffffu);
-        pl[off + so.plane_stride] = (uint16_t)(l & 0xffffu);
-        pl[off + 2 * so.plane_stride] = (uint16_t)(h >> 16);
-        pl[off + 3 * so.plane_stride] = (uint16_t)(l >> 16);
+        pl[off + so.lo_stride] = (uint16_t)(l & 0xffffu);
+        pl[off + so.im_stride] = (uint16_t)(h >> 16);
+        pl[off + so.im_stride + so.lo_stride] = (uint16_t)(l >> 16);
         if (so.extra == kSplitNegIm) { // -x: the sign bit of each piece flipped
             pl[off + 4 * so.plane_stride] = (uint16_t)((h >> 16) ^ 0x8000u);
             pl[off + 5 * so.plane_stride] = (uint16_t)((l >> 16) ^ 0x8000u);
@@ -283,9 +294,9 @@ __device__ __forceinline__ void WriteSplit(const SplitOut &so, uint64_t o, float
     float rh = RoundTf32(re), ih = RoundTf32(im);
     float rl = RoundTf32(re - rh), il = RoundTf32(im - ih);
     planes[off] = rh;
-    planes[off + so.plane_stride] = rl;
-    planes[off + 2 * so.plane_stride] = ih;
-    planes[off + 3 * so.plane_stride] = il;
+    planes[off + so.lo_stride] = rl;
+    planes[off + so.im_stride] = ih;
+    planes[off + so.im_stride + so.lo_stride] = il;
     if (so.extra == kSplitNegIm) {
         planes[off + 4 * so.plane_stride] = -ih;
         planes[off + 5 * so.plane_stride] = -il;
@@ -757,7 +768,7 @@ struct SplitStore {
         // instruction bound).
         uint64_t row = off >> so.cols_log2;
         uint64_t col = off & (so.cols - 1);
-        uint64_t base = row * so.pitch + col;
+        const uint64_t base = SplitOffset(so, row, col);
         float2 a = make_float2(__uint_as_float(v[0].x), __uint_as_float(v[0].y));
         float2 b = make_float2(__uint_as_float(v[1].x), __uint_as_float(v[1].y));
         const float sc = SplitScale(so);
@@ -770,9 +781,9 @@ struct SplitStore {
             Split16x2(so, ar, br, rh, rl);
             Split16x2(so, ai, bi, ih, il);
             *reinterpret_cast<uint32_t *>(pl + base) = rh;
-            *reinterpret_cast<uint32_t *>(pl + base + so.plane_stride) = rl;
-            *reinterpret_cast<uint32_t *>(pl + base + 2 * so.plane_stride) = ih;
-            *reinterpret_cast<uint32_t *>(pl + base + 3 * so.plane_stride) = il;
+            *reinterpret_cast<uint32_t *>(pl + base + so.lo_stride) = rl;
+            *reinterpret_cast<uint32_t *>(pl + base + so.im_stride) = ih;
+            *reinterpret_cast<uint32_t *>(pl + base + so.im_stride + so.lo_stride) = il;
             if (so.extra == kSplitNegIm) { // -x: the sign bit of each piece flipped
                 *reinterpret_cast<uint32_t *>(pl + base + 4 * so.plane_stride) = ih ^ 0x80008000u;
                 *reinterpret_cast<uint32_t *>(pl + base + 5 * so.plane_stride) = il ^ 0x80008000u;
@@ -793,9 +804,9 @@ struct SplitStore {
         float2 ih = make_float2(aih, bih);
         float2 il = make_float2(RoundTf32(ai - aih), RoundTf32(bi - bih));
         *reinterpret_cast<float2 *>(planes + base) = rh;
-        *reinterpret_cast<float2 *>(planes + base + so.plane_stride) = rl;
-        *reinterpret_cast<float2 *>(planes + base + 2 * so.plane_stride) = ih;
-        *reinterpret_cast<float2 *>(planes + base + 3 * so.plane_stride) = il;
+        *reinterpret_cast<float2 *>(planes + base + so.lo_stride) = rl;
+        *reinterpret_cast<float2 *>(planes + base + so.im_stride) = ih;
+        *reinterpret_cast<float2 *>(planes + base + so.im_stride + so.lo_stride) = il;
         if (so.extra == kSplitNegIm) {
             *reinterpret_cast<float2 *>(planes + base + 4 * so.plane_stride) =
                 make_float2(-ih.x, -ih.y);
@@ -1077,7 +1088,7 @@ int PermuteSplitTf32Batched(const void *in, float *planes, uint64_t batch, int r
 int PermuteSplitPlanes(const void *in, void *planes, uint64_t batch, int rank,
                        const uint64_t *shape, const int32_t *perm, uint64_t rows, uint64_t cols,
                        uint64_t pitch, uint64_t plane_stride, int scale_exp, SplitFormat fmt,
-                       int extra, cudaStream_t stream, const int *e_max_dev)
+                       int extra, cudaStream_t stream, const int *e_max_dev, bool paired)
 {
     JETGPU_REQUIRE(extra == kSplitNone || extra == kSplitNegIm || extra == kSplitSum,
                    "unknown extra plane pair");
@@ -1103,6 +1114,12 @@ int PermuteSplitPlanes(const void *in, void *planes, uint64_t batch, int rank,
     so.bf16 = fmt == SplitFormat::kBf16 ? 1 : 0;
     so.fp16 = fmt == SplitFormat::kFp16 ? 1 : 0;
     so.e_max_dev = e_max_dev;
+    JETGPU_REQUIRE(!paired || (extra == kSplitNone && cols % SplitPairWords(fmt) == 0 &&
+                               pitch >= 2 * cols),
+                   "paired planes need whole blocks");
+    so.pair_log2 = paired ? Log2(SplitPairWords(fmt)) : 0;
+    so.lo_stride = paired ? SplitPairWords(fmt) : plane_stride;
+    so.im_stride = paired ? plane_stride : 2 * plane_stride;
     so.cols_log2 = IsPow2(cols) ? Log2(cols) : -1;
     so.narrow = s.size * batch < (1ull << 32) ? 1 : 0;
     so.cols_magic = so.cols_shift = 0;
