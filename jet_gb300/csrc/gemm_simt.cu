@@ -548,6 +548,52 @@ __global__ void reduce_partials_warp(const typename C2<T>::type *__restrict__ pa
     }
 }
 
+// The sums of a jetgpu_contract product's k ranges, complex64, in range order.
+// FP64 adds and conversions bound the kernel above on this GPU (2^18 outputs of
+// nine ranges 24 us, their 19 MB in L2): here the running sum is a pair of
+// FP32 values, the second holding the exact rounding errors of the first's
+// adds (Knuth's two-sum), so a sum is rounded once at the end, as in FP64.
+struct PairSum {
+    float s = 0, e = 0;
+    __device__ __forceinline__ void add(float x)
+    {
+        const float t = s + x;
+        const float b = t - s;
+        e += (s - (t - b)) + (x - b);
+        s = t;
+    }
+    // An infinite or NaN sum has no error to add.
+    __device__ __forceinline__ float value() const { return isfinite(s) ? s + e : s; }
+};
+
+__global__ void __launch_bounds__(256)
+    sum_partials_kernel(const float2 *__restrict__ part, float2 *__restrict__ out, int64_t len,
+                        int64_t S)
+{
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        PairSum re, im;
+        int64_t s = 0;
+        for (; s + 4 <= S; s += 4) {
+            float2 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                v[u] = part[(s + u) * len + i];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                re.add(v[u].x);
+                im.add(v[u].y);
+            }
+        }
+        for (; s < S; ++s) {
+            const float2 v = part[s * len + i];
+            re.add(v.x);
+            im.add(v.y);
+        }
+        out[i] = make_float2(re.value(), im.value());
+    }
+}
+
 // Sums S partial results of `len` elements each into out (a fixed order).
 template <typename T>
 int ReducePartials(const typename C2<T>::type *part, typename C2<T>::type *out, int64_t len,
@@ -894,8 +940,9 @@ int MultiplyPlainBatched(const void *A, const void *B, void *C, uint64_t batch, 
 
 int SumPartials(const void *part, void *out, uint64_t len, uint64_t splits, cudaStream_t stream)
 {
-    return ReducePartials<float>((const float2 *)part, (float2 *)out, (int64_t)len,
-                                 (int64_t)splits, stream);
+    sum_partials_kernel<<<GridFor((len + 255) / 256, 8), 256, 0, stream>>>(
+        (const float2 *)part, (float2 *)out, (int64_t)len, (int64_t)splits);
+    return CheckLaunch("sum_partials_kernel");
 }
 
 size_t MultiplyPlainWorkspace(uint64_t m, uint64_t n, uint64_t k, int dtype)
