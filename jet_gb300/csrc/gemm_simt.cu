@@ -228,6 +228,10 @@ template <typename T> struct KahanSum {
     }
 };
 
+// Groups of four products whose loads a thread of the vector kernels issues
+// at once (32 eight-byte or 16 sixteen-byte loads).
+template <typename T> constexpr int kVectorGroups = sizeof(T) == 4 ? 4 : 2;
+
 // y[b, m] (+ partial s) = sum_{k in chunk s} A_b[m, k] x_b[k]. A CTA of 8
 // warps covers `rows` rows (8, 4, 2 or 1) with 8 / rows warps per row, which
 // interleave the row's k chunk, so few rows still keep every warp streaming.
@@ -260,6 +264,29 @@ __global__ void __launch_bounds__(256)
         // carries one rounding of the plain FMA chain).
         const int64_t step = wpr * 32;
         int64_t k = k_begin + part * 32 + lane;
+        // Several such groups' loads at once: a split's few rows leave most
+        // SMs with one CTA, which would wait out a memory latency per group.
+        constexpr int G = kVectorGroups<T>;
+        for (; k + (4 * G - 1) * step < k_end; k += 4 * G * step) {
+            V a[4 * G], xv[4 * G];
+#pragma unroll
+            for (int u = 0; u < 4 * G; ++u) {
+                a[u] = A[m * K + k + u * step];
+                xv[u] = x[k + u * step];
+            }
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                T re = a[4 * g].x * xv[4 * g].x - a[4 * g].y * xv[4 * g].y;
+                T im = a[4 * g].x * xv[4 * g].y + a[4 * g].y * xv[4 * g].x;
+#pragma unroll
+                for (int u = 4 * g + 1; u < 4 * g + 4; ++u) {
+                    re = fma(a[u].x, xv[u].x, fma(-a[u].y, xv[u].y, re));
+                    im = fma(a[u].x, xv[u].y, fma(a[u].y, xv[u].x, im));
+                }
+                sr.add(re);
+                si.add(im);
+            }
+        }
         for (; k + 3 * step < k_end; k += 4 * step) {
             V a[4], xv[4];
 #pragma unroll
@@ -332,8 +359,30 @@ __global__ void __launch_bounds__(256)
     out += (s * gridDim.z + b) * N;
     KahanSum<T> sr, si;
     if (n < N) {
-        // Four products per compensated add (see gemv_rows_kernel).
+        // Four products per compensated add, several groups' loads at once
+        // (see gemv_rows_kernel).
         int64_t k = k_begin + tk;
+        constexpr int G = kVectorGroups<T>;
+        for (; k + (4 * G - 1) * (int64_t)tk_count < k_end; k += 4 * G * (int64_t)tk_count) {
+            V a[4 * G], v[4 * G];
+#pragma unroll
+            for (int u = 0; u < 4 * G; ++u) {
+                a[u] = x[k + u * tk_count];
+                v[u] = B[(k + u * tk_count) * N + n];
+            }
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                T re = a[4 * g].x * v[4 * g].x - a[4 * g].y * v[4 * g].y;
+                T im = a[4 * g].x * v[4 * g].y + a[4 * g].y * v[4 * g].x;
+#pragma unroll
+                for (int u = 4 * g + 1; u < 4 * g + 4; ++u) {
+                    re = fma(a[u].x, v[u].x, fma(-a[u].y, v[u].y, re));
+                    im = fma(a[u].x, v[u].y, fma(a[u].y, v[u].x, im));
+                }
+                sr.add(re);
+                si.add(im);
+            }
+        }
         for (; k + 3 * (int64_t)tk_count < k_end; k += 4 * (int64_t)tk_count) {
             V a[4], v[4];
 #pragma unroll

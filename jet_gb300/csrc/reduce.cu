@@ -96,7 +96,23 @@ struct SliceParams {
     uint64_t out_size;
     uint64_t first_value;
     uint64_t total;                   // n_values * out_size
+    int narrow;                       // total, dims and value strides below 2^32
 };
+
+// Input offset of element o of slice value v, with divisions of width U.
+template <typename U> __device__ __forceinline__ uint64_t SliceSrc(const SliceParams &p, U v, U o)
+{
+    uint64_t src = 0;
+    for (int j = 0; j < p.n_axes; ++j)
+        src += (uint64_t)((v / (U)p.value_stride[j]) % (U)p.fixed_dim[j]) * p.fixed_stride[j];
+    for (int j = p.free_rank - 1; j >= 0; --j) {
+        const U d = (U)p.free_dims[j];
+        const U q = o / d;
+        src += (uint64_t)(o - q * d) * p.free_strides[j];
+        o = q;
+    }
+    return src;
+}
 
 template <typename E>
 __global__ void slice_gather_kernel(const __grid_constant__ SliceParams p,
@@ -108,19 +124,17 @@ __global__ void slice_gather_kernel(const __grid_constant__ SliceParams p,
     const uint64_t first = first_dev ? *first_dev : p.first_value;
     for (uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
          idx < p.total; idx += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t s = idx / p.out_size;
-        uint64_t o = idx - s * p.out_size;
-        const uint64_t v = first + s;
-        uint64_t src = 0;
-        for (int j = 0; j < p.n_axes; ++j)
-            src += ((v / p.value_stride[j]) % p.fixed_dim[j]) * p.fixed_stride[j];
-        for (int j = p.free_rank - 1; j >= 0; --j) {
-            const uint64_t d = p.free_dims[j];
-            const uint64_t q = o / d;
-            src += (o - q * d) * p.free_strides[j];
-            o = q;
+        // A leaf's gather is a chain of divisions: in 32 bits where sizes and
+        // slice values allow it.
+        const uint64_t last = first + p.total / p.out_size;
+        if (p.narrow && last < (1ull << 32)) {
+            const uint32_t i = (uint32_t)idx, n = (uint32_t)p.out_size;
+            const uint32_t s = i / n;
+            out[idx] = in[SliceSrc<uint32_t>(p, (uint32_t)first + s, i - s * n)];
+            continue;
         }
-        out[idx] = in[src];
+        const uint64_t s = idx / p.out_size;
+        out[idx] = in[SliceSrc<uint64_t>(p, first + s, idx - s * p.out_size)];
     }
 }
 
@@ -406,6 +420,10 @@ static int SliceGatherImpl(const void *in, int rank, const uint64_t *shape, int 
         }
     p.first_value = first_value;
     p.total = p.out_size * n_values;
+    p.narrow = p.total < (1ull << 32) ? 1 : 0;
+    for (int j = 0; j < n_axes; ++j)
+        if ((p.value_stride[j] | p.fixed_dim[j]) >> 32)
+            p.narrow = 0;
     if (p.total == 0)
         return JETGPU_OK;
     JETGPU_REQUIRE(in && out, "null pointer");
