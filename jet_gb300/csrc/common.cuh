@@ -292,6 +292,13 @@ int MultiplyPlain(const void *A, const void *B, void *C, uint64_t m,
 
 size_t MultiplyPlainWorkspace(uint64_t m, uint64_t n, uint64_t k, int dtype);
 
+// MultiplyPlain for a jetgpu_contract call: may cut k of a matrix product into
+// more ranges when the workspace holds MultiplySingleWorkspace bytes.
+int MultiplySingle(const void *A, const void *B, void *C, uint64_t m, uint64_t n, uint64_t k,
+                   int dtype, int scale_exp, void *workspace, size_t ws_bytes,
+                   cudaStream_t stream);
+size_t MultiplySingleWorkspace(uint64_t m, uint64_t n, uint64_t k, int dtype);
+
 // Tensor-core 3xTF32 complex product of planar operands (see gemm_tc.cu).
 int GemmTf32x3Planar(const float *a_planes, const float *b_planes, void *C,
                      uint64_t m, uint64_t n, uint64_t k, uint64_t kpitch,

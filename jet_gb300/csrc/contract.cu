@@ -408,7 +408,8 @@ size_t FormWorkspace(uint64_t batch, int a_rank, const uint64_t *a_shape, const 
         ws += AlignUp(p.ba * m * k * eb);
     if (!IsIdentity(b_rank, b_perm))
         ws += AlignUp(p.bb * k * n * eb);
-    ws += AlignUp(batch == 1 ? MultiplyPlainWorkspace(m, n, k, dtype)
+    ws += AlignUp(batch == 1 ? (single ? MultiplySingleWorkspace(m, n, k, dtype)
+                                       : MultiplyPlainWorkspace(m, n, k, dtype))
                              : MultiplyPlainBatchedWorkspace(batch, m, n, k, dtype));
     return ws;
 }
@@ -489,6 +490,9 @@ int ContractForm(uint64_t batch, const void *A, int a_rank, const uint64_t *a_sh
         btp = ws;
         ws += AlignUp(p.bb * k * n * eb);
     }
+    if (batch == 1 && single_ws > 0)
+        return MultiplySingle(at, btp, C, m, n, k, dtype, scale_a + scale_b, ws,
+                              single_ws - (size_t)(ws - static_cast<uint8_t *>(workspace)), st);
     if (batch == 1) {
         const size_t vec_ws = MultiplyPlainWorkspace(m, n, k, dtype);
         return MultiplyPlain(at, btp, C, m, n, k, dtype, scale_a + scale_b, ws, vec_ws, st);

@@ -728,7 +728,7 @@ constexpr GemmTile kTilesC64[] = {
     {32, 32, 83, 61},   // 2 x 2
 };
 constexpr int kNumTilesC64 = sizeof(kTilesC64) / sizeof(kTilesC64[0]);
-constexpr GemmTile kTileC128 = {32, 32, 0, 0};
+constexpr GemmTile kTileC128 = {32, 32, 2100, 2100};
 
 inline int64_t CeilDiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
@@ -739,12 +739,44 @@ inline double TileClocks(const GemmTile &t, int64_t M, int64_t N, int64_t z)
     return std::max(t.alone, (double)per_sm * t.shared);
 }
 
+// k ranges of one product (jetgpu_contract): products of few tiles leave SMs
+// idle, so k is cut while the busiest SM then finishes sooner, adding the
+// ranges' sums (a launch, and their bytes through L2) included. At least 64 k
+// a range, and none below 256: steps of k <= 64 add in one order everywhere
+// (grouped launches and skinny kernels give the same bits).
+constexpr int64_t kSingleMinK = 256;
+constexpr double kReduceClocks = 6000.0; // a launch and its latency
+constexpr double kReduceBytes = 2000.0;  // partial sums per clock
+
+template <typename T> int64_t SingleSplits(int64_t M, int64_t N, int64_t K);
+
 inline int PickTileC64(int64_t M, int64_t N, int64_t z)
 {
     int best = 0;
     for (int i = 1; i < kNumTilesC64; ++i)
         if (TileClocks(kTilesC64[i], M, N, z) < TileClocks(kTilesC64[best], M, N, z))
             best = i;
+    return best;
+}
+
+template <typename T> int64_t SingleSplits(int64_t M, int64_t N, int64_t K)
+{
+    if (K < kSingleMinK || SmCount() < 1)
+        return 1;
+    int64_t best = 1;
+    double least = 0;
+    for (int64_t S = 1; K / S >= kSingleMinK / 4; S *= 2) {
+        const double bytes = (double)S * M * N * 2 * sizeof(T);
+        if (S > 1 && bytes > (double)(32 << 20))
+            break;
+        const GemmTile &t = sizeof(T) == 4 ? kTilesC64[PickTileC64(M, N, S)] : kTileC128;
+        const double clocks = TileClocks(t, M, N, S) * (double)CeilDiv(K, S) +
+                              (S > 1 ? kReduceClocks + bytes / kReduceBytes : 0.0);
+        if (S == 1 || clocks < least) {
+            best = S;
+            least = clocks;
+        }
+    }
     return best;
 }
 
@@ -859,7 +891,7 @@ int MultiplyVectorT(const typename C2<T>::type *A, const typename C2<T>::type *B
 template <typename T>
 int GemmT(const typename C2<T>::type *A, const typename C2<T>::type *B, typename C2<T>::type *C,
           int64_t batch, int64_t sa, int64_t sb, int64_t M, int64_t N, int64_t K, T scale,
-          void *ws, size_t ws_bytes, cudaStream_t stream)
+          void *ws, size_t ws_bytes, cudaStream_t stream, int64_t single_splits = 0)
 {
     using V = typename C2<T>::type;
     const size_t need = VectorWorkspace<T>(batch, M, N, K);
@@ -885,7 +917,8 @@ int GemmT(const typename C2<T>::type *A, const typename C2<T>::type *B, typename
             return rc;
         return ReducePartials<T>(dst, C, batch * M * N, S, stream);
     }
-    const int64_t S = (need > 0 && ws != nullptr && ws_bytes >= need)
+    const int64_t S = single_splits > 0 ? single_splits
+                      : (need > 0 && ws != nullptr && ws_bytes >= need)
                           ? BatchedSplits<T>(batch, M, N, K)
                           : 1;
     const int64_t kchunk = (K + S - 1) / S;
@@ -925,6 +958,8 @@ int GemmT(const typename C2<T>::type *A, const typename C2<T>::type *B, typename
     int rc = CheckLaunch("gemm_kernel");
     if (rc || S == 1)
         return rc;
+    if (std::is_same<T, float>::value && single_splits > 0)
+        return SumPartials(dst, C, (uint64_t)(M * N), (uint64_t)S, stream);
     return ReducePartials<T>(dst, C, batch * M * N, S, stream);
 }
 
@@ -992,6 +1027,45 @@ int SumPartials(const void *part, void *out, uint64_t len, uint64_t splits, cuda
     sum_partials_kernel<<<GridFor((len + 255) / 256, 8), 256, 0, stream>>>(
         (const float2 *)part, (float2 *)out, (int64_t)len, (int64_t)splits);
     return CheckLaunch("sum_partials_kernel");
+}
+
+namespace {
+
+// The k ranges jetgpu_contract cuts a matrix product into (1: its plain path).
+int64_t SingleRanges(uint64_t m, uint64_t n, uint64_t k, int dtype)
+{
+    int mt, nt;
+    SmallTile((int64_t)m, (int64_t)n, (int64_t)k, mt, nt);
+    if (m < 2 || n < 2 || k == 0 || mt)
+        return 1;
+    return dtype == JETGPU_C128 ? SingleSplits<double>((int64_t)m, (int64_t)n, (int64_t)k)
+                                : SingleSplits<float>((int64_t)m, (int64_t)n, (int64_t)k);
+}
+
+} // namespace
+
+size_t MultiplySingleWorkspace(uint64_t m, uint64_t n, uint64_t k, int dtype)
+{
+    const int64_t S = SingleRanges(m, n, k, dtype);
+    return std::max(MultiplyPlainWorkspace(m, n, k, dtype),
+                    S > 1 ? (size_t)S * m * n * ElemBytes(dtype) : 0);
+}
+
+int MultiplySingle(const void *A, const void *B, void *C, uint64_t m, uint64_t n, uint64_t k,
+                   int dtype, int scale_exp, void *workspace, size_t ws_bytes,
+                   cudaStream_t stream)
+{
+    const int64_t S = SingleRanges(m, n, k, dtype);
+    const size_t bytes = (size_t)S * m * n * ElemBytes(dtype);
+    if (S < 2 || workspace == nullptr || ws_bytes < bytes)
+        return MultiplyPlain(A, B, C, m, n, k, dtype, scale_exp, workspace, ws_bytes, stream);
+    if (dtype == JETGPU_C128)
+        return GemmT<double>((const double2 *)A, (const double2 *)B, (double2 *)C, 1, 0, 0,
+                             (int64_t)m, (int64_t)n, (int64_t)k, ldexp(1.0, scale_exp), workspace,
+                             bytes, stream, S);
+    return GemmT<float>((const float2 *)A, (const float2 *)B, (float2 *)C, 1, 0, 0, (int64_t)m,
+                        (int64_t)n, (int64_t)k, (float)ldexp(1.0, scale_exp), workspace, bytes,
+                        stream, S);
 }
 
 size_t MultiplyPlainWorkspace(uint64_t m, uint64_t n, uint64_t k, int dtype)
