@@ -431,14 +431,21 @@ __global__ void __launch_bounds__(256)
 // where gemm_kernel's 32 x 64 tile is three quarters empty and streams 8 k per
 // pass with few loads in flight (1.06 ms, 0.76 TB/s). Here one CTA per
 // (k range, batch item):
-//  * the A (MT x KC, stored k-major under an XOR swizzle) and B (KC x NT)
-//    tiles of the range come in by cp.async, double-buffered, elements past
-//    M, N or the range zero-filled; KC = 32 (complex64) or 16 (complex128),
-//    so each warp has four (two) k per tile between barriers;
+//  * the A (MT x KC, stored k-major) and B (KC x NT) tiles of the range come in
+//    by cp.async, double-buffered, elements past M, N or the range zero-filled;
+//    KC = 32 (complex64) or 16 (complex128), so each warp has four (two) k per
+//    tile between barriers;
 //  * the 8 warps split every tile, each lane accumulating an
-//    (MT / 4) x (NT / 8) block, so each warp covers the whole output;
+//    (MT / 4) x (NT / 8) block, so each warp covers the whole output. MT x NT is
+//    the smallest of 4 x 8, 8 x 16, 16 x 16, 16 x 32 and 32 x 16 that holds the
+//    output (2 x 2 outputs in 16 x 32 tiles cost as much as 512); which k a warp
+//    adds does not depend on it;
 //  * the warps' sums are added in warp order in shared memory and the k
 //    ranges' in the workspace by reduce_partials: a fixed order.
+// Bound by FMA issue at 16 x 32 (complex128: by the FP64 pipe), by its barriers
+// below. 16 x 32 x 2^21 complex64: 361 -> 253 us with padded rows in the place of
+// an XOR per load and with pointers that advance; 2 x 2 x 2^21 350 -> 60;
+// complex128 4 x 8 x 2^17 547 -> 49.
 template <typename T, int MT, int NT>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
     gemm_small_kernel(const typename C2<T>::type *__restrict__ A,
@@ -448,9 +455,16 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
 {
     using V = typename C2<T>::type;
     constexpr int TR = MT / 4, TC = NT / 8;
+    static_assert((TR == 1 || TR % 2 == 0) && (TC == 1 || TC % 2 == 0), "one or whole pairs");
     constexpr int kSmallKC = sizeof(T) == 4 ? 32 : 16;
     constexpr int NS = 2; // stages (three measured 5 % slower: occupancy, not latency, binds)
-    __shared__ __align__(16) V As[NS][kSmallKC * MT];
+    constexpr int G = 16 / sizeof(V); // elements per 16-byte shared-memory load
+    // Copies per thread (the smallest tiles leave some threads without).
+    constexpr int AP = (MT * kSmallKC + 255) / 256, BP = (NT * kSmallKC + 255) / 256;
+    struct alignas(16) Pack {
+        V v[G];
+    };
+    __shared__ __align__(16) V As[NS][kSmallKC][MT + G];
     __shared__ __align__(16) V Bs[NS][kSmallKC][NT];
     __shared__ V red[MT * NT];
     const int64_t s = blockIdx.x, bz = blockIdx.z, batch = gridDim.z;
@@ -463,20 +477,33 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rg = lane >> 3, cg = lane & 7;
 
-    auto load = [&](int st, int64_t t) {
-        const int64_t k0 = k_begin + t * kSmallKC;
-        for (int e = tid; e < MT * kSmallKC; e += 256) {
-            const int i = e / kSmallKC, kk = e % kSmallKC;
-            const bool ok = i < M && k0 + kk < k_end;
-            CpAsyncElem(&As[st][kk * MT + (i ^ (kk & (MT - 1)))], ok ? A + i * K + k0 + kk : A,
-                        ok);
+    // This thread's copies of a tile: elements (i, kk) of A, (kk, j) of B, at
+    // pointers that advance with the tiles.
+    const int a_kk = tid % kSmallKC, a_i = tid / kSmallKC;
+    const int b_j = tid % NT, b_kk = tid / NT;
+    const V *pa = A + a_i * K + k_begin + a_kk;
+    const V *pb = B + (k_begin + b_kk) * N + b_j;
+    const int64_t a_step = (int64_t)(256 / kSmallKC) * K, b_step = (int64_t)(256 / NT) * N;
+    int64_t left = k_end - k_begin; // k from the next tile to load on
+    auto load = [&](int st) {
+#pragma unroll
+        for (int q = 0; q < AP; ++q) {
+            const int i = a_i + q * (256 / kSmallKC);
+            const bool ok = i < M && a_kk < left;
+            if (MT * kSmallKC >= 256 || i < MT)
+                CpAsyncElem(&As[st][a_kk][i], ok ? pa + q * a_step : A, ok);
         }
-        for (int e = tid; e < kSmallKC * NT; e += 256) {
-            const int kk = e / NT, j = e % NT;
-            const bool ok = j < N && k0 + kk < k_end;
-            CpAsyncElem(&Bs[st][kk][j], ok ? B + (k0 + kk) * N + j : B, ok);
+#pragma unroll
+        for (int q = 0; q < BP; ++q) {
+            const int kk = b_kk + q * (256 / NT);
+            const bool ok = b_j < N && kk < left;
+            if (NT * kSmallKC >= 256 || kk < kSmallKC)
+                CpAsyncElem(&Bs[st][kk][b_j], ok ? pb + q * b_step : B, ok);
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
+        pa += kSmallKC;
+        pb += (int64_t)kSmallKC * N;
+        left -= kSmallKC;
     };
 
     V acc[TR][TC];
@@ -487,16 +514,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
             acc[r][c] = V{0, 0};
     // Every iteration commits one group (empty past the last tile), so
     // wait_group NS - 1 always means "tile t has landed".
-    for (int q = 0; q < NS - 1; ++q) {
-        if (q < tiles)
-            load(q, q);
-        else
-            asm volatile("cp.async.commit_group;\n" ::: "memory");
-    }
+    if (tiles > 0)
+        load(0);
+    int st = 0;
     for (int64_t t = 0; t < tiles; ++t) {
-        const int st = (int)(t % NS);
-        if (t + NS - 1 < tiles)
-            load((int)((t + NS - 1) % NS), t + NS - 1);
+        if (t + 1 < tiles)
+            load(st ^ 1);
         else
             asm volatile("cp.async.commit_group;\n" ::: "memory");
         asm volatile("cp.async.wait_group %0;\n" ::"n"(NS - 1) : "memory");
@@ -505,22 +528,43 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
         for (int kk = warp; kk < kSmallKC; kk += 8) {
             V a[TR], b[TC];
 #pragma unroll
-            for (int r = 0; r < TR; ++r)
-                a[r] = As[st][kk * MT + ((rg * TR + r) ^ (kk & (MT - 1)))];
+            for (int r = 0; r < TR; r += G) {
+                if constexpr (TR % G != 0) {
+                    a[r] = As[st][kk][rg * TR + r];
+                    continue;
+                }
+                const Pack w = *reinterpret_cast<const Pack *>(&As[st][kk][rg * TR + r]);
 #pragma unroll
-            for (int c = 0; c < TC; ++c)
-                b[c] = Bs[st][kk][cg * TC + c];
+                for (int u = 0; u < G; ++u)
+                    a[r + u] = w.v[u];
+            }
 #pragma unroll
-            for (int r = 0; r < TR; ++r)
+            for (int c = 0; c < TC; c += G) {
+                if constexpr (TC % G != 0) {
+                    b[c] = Bs[st][kk][cg * TC + c];
+                    continue;
+                }
+                const Pack w = *reinterpret_cast<const Pack *>(&Bs[st][kk][cg * TC + c]);
+#pragma unroll
+                for (int u = 0; u < G; ++u)
+                    b[c + u] = w.v[u];
+            }
+#pragma unroll
+            for (int r = 0; r < TR; ++r) {
 #pragma unroll
                 for (int c = 0; c < TC; ++c) {
                     acc[r][c].x = fma(a[r].x, b[c].x, acc[r][c].x);
-                    acc[r][c].x = fma(-a[r].y, b[c].y, acc[r][c].x);
                     acc[r][c].y = fma(a[r].x, b[c].y, acc[r][c].y);
+                }
+#pragma unroll
+                for (int c = 0; c < TC; ++c) {
+                    acc[r][c].x = fma(-a[r].y, b[c].y, acc[r][c].x);
                     acc[r][c].y = fma(a[r].y, b[c].x, acc[r][c].y);
                 }
+            }
         }
         __syncthreads(); // the next load reuses this stage
+        st ^= 1;
     }
     for (int w = 0; w < 8; ++w) {
         if (warp == w) {
@@ -690,7 +734,15 @@ inline void SmallTile(int64_t M, int64_t N, int64_t K, int &mt, int &nt)
     mt = nt = 0;
     if (K < 2048 || M < 2 || N < 2)
         return;
-    if (M <= 16 && N <= 32) {
+    if (M <= 4 && N <= 8) {
+        mt = 4;
+        nt = 8;
+    } else if (M <= 8 && N <= 16) {
+        mt = 8;
+        nt = 16;
+    } else if (M <= 16 && N <= 16) {
+        mt = nt = 16;
+    } else if (M <= 16 && N <= 32) {
         mt = 16;
         nt = 32;
     } else if (M <= 32 && N <= 16) {
@@ -906,12 +958,19 @@ int GemmT(const typename C2<T>::type *A, const typename C2<T>::type *B, typename
         const int64_t kchunk = (K + S - 1) / S;
         V *dst = S > 1 ? (V *)ws : C;
         const dim3 grid((unsigned)S, 1u, (unsigned)batch);
-        if (mt == 16)
-            gemm_small_kernel<T, 16, 32><<<grid, 256, 0, stream>>>(A, B, dst, M, N, K, scale, sa,
-                                                                   sb, kchunk);
+        const auto launch = [&](auto kernel) {
+            kernel<<<grid, 256, 0, stream>>>(A, B, dst, M, N, K, scale, sa, sb, kchunk);
+        };
+        if (mt == 4)
+            launch(gemm_small_kernel<T, 4, 8>);
+        else if (mt == 8)
+            launch(gemm_small_kernel<T, 8, 16>);
+        else if (mt == 16 && nt == 16)
+            launch(gemm_small_kernel<T, 16, 16>);
+        else if (mt == 16)
+            launch(gemm_small_kernel<T, 16, 32>);
         else
-            gemm_small_kernel<T, 32, 16><<<grid, 256, 0, stream>>>(A, B, dst, M, N, K, scale, sa,
-                                                                   sb, kchunk);
+            launch(gemm_small_kernel<T, 32, 16>);
         int rc = CheckLaunch("gemm_small_kernel");
         if (rc || S == 1)
             return rc;
