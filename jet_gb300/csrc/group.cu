@@ -22,8 +22,10 @@
 // all loads of eight k issued before any arithmetic: no staging, no barrier.
 // Through staged 32 x 32 x 32 slices, mostly padding, the smallest launch took
 // 7.5 us. Tiles of more work are staged in shared memory, 2 x 2 outputs a
-// thread. The launch uses programmatic stream serialisation, so that a chain
-// of levels overlaps each launch with the end of the one before.
+// thread. Whole k in one stage (64 of complex64) measured the same.
+// The launch uses programmatic stream serialisation, so that a chain of levels
+// overlaps each launch with the end of the one before: a gradient's replay
+// (53 grouped launches) 1,477 -> 1,459 us, 81 qutrit slices 4,498 -> 4,475 us.
 #include "common.cuh"
 
 namespace jetgpu {
@@ -66,8 +68,11 @@ __global__ void __launch_bounds__(kGThreads)
     __shared__ uint64_t warp_sum[kGThreads / 32];
     __shared__ V As[kGK][kGT + 1];
     __shared__ V Bs[kGK][kGT + 1];
-    // Every memory access follows this wait for the kernel before; the next
-    // launch may start once every CTA is past it.
+    // Every access to operands and outputs follows this wait for the kernel
+    // before; the next launch may start once every CTA is past it. The task
+    // table may be read earlier: a launch starts early only behind another
+    // grouped launch, which writes nothing but its outputs, and only once all
+    // that came before that one has ended.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // First tile of every task: thread t reads task t's tile count, then an
