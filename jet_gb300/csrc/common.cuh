@@ -299,6 +299,14 @@ int MultiplySingle(const void *A, const void *B, void *C, uint64_t m, uint64_t n
                    cudaStream_t stream);
 size_t MultiplySingleWorkspace(uint64_t m, uint64_t n, uint64_t k, int dtype);
 
+// A small output over a long k read from the operands' own layouts (power-of-2
+// extents), arguments as ContractForm's; `taken` false: not such a product,
+// nothing was done. Cuts k into as many ranges as `workspace` has room for.
+int ClosingContract(const void *A, int a_rank, const uint64_t *a_shape, const int32_t *a_perm,
+                    const void *B, int b_rank, const uint64_t *b_shape, const int32_t *b_perm,
+                    void *C, uint64_t m, uint64_t n, uint64_t k, int dtype, int scale_exp,
+                    void *workspace, size_t ws_bytes, cudaStream_t stream, bool &taken);
+
 // Tensor-core 3xTF32 complex product of planar operands (see gemm_tc.cu).
 int GemmTf32x3Planar(const float *a_planes, const float *b_planes, void *C,
                      uint64_t m, uint64_t n, uint64_t k, uint64_t kpitch,

@@ -472,6 +472,16 @@ int ContractForm(uint64_t batch, const void *A, int a_rank, const uint64_t *a_sh
         return SkinnyContract(batch, A, a_rank, a_shape, a_perm, a_batched, B, b_rank, b_shape,
                               b_perm, b_batched, C, m, n, k, dtype, scale_a + scale_b, st);
     int rc;
+    // Two operands in order already go to the packed kernel, which reads whole
+    // rows; any transpose costs more than reading in place.
+    if (batch == 1 && single_ws > 0 && k > 0 &&
+        (!IsIdentity(a_rank, a_perm) || !IsIdentity(b_rank, b_perm))) {
+        bool taken;
+        rc = ClosingContract(A, a_rank, a_shape, a_perm, B, b_rank, b_shape, b_perm, C, m, n, k,
+                             dtype, scale_a + scale_b, workspace, single_ws, st, taken);
+        if (taken)
+            return rc;
+    }
     const size_t eb = ElemBytes(dtype);
     const void *at = A;
     const void *btp = B;

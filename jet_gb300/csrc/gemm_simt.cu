@@ -13,6 +13,8 @@
 //    (deterministic).
 #include <algorithm>
 #include <type_traits>
+#include <utility>
+#include <vector>
 
 #include "common.cuh"
 
@@ -425,6 +427,87 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// One k of a small output's tile: lane (rg, cg) adds its TR x TC block, `a` and
+// `b` at its values of the k's rows.
+template <typename T, int TR, int TC>
+__device__ __forceinline__ void SmallMac(typename C2<T>::type (&acc)[TR][TC],
+                                         const typename C2<T>::type *as,
+                                         const typename C2<T>::type *bs)
+{
+    using V = typename C2<T>::type;
+    constexpr int G = 16 / sizeof(V); // elements per 16-byte shared-memory load
+    struct alignas(16) Pack {
+        V v[G];
+    };
+    V a[TR], b[TC];
+#pragma unroll
+    for (int r = 0; r < TR; r += G) {
+        if constexpr (TR % G != 0) {
+            a[r] = as[r];
+            continue;
+        }
+        const Pack w = *reinterpret_cast<const Pack *>(as + r);
+#pragma unroll
+        for (int u = 0; u < G; ++u)
+            a[r + u] = w.v[u];
+    }
+#pragma unroll
+    for (int c = 0; c < TC; c += G) {
+        if constexpr (TC % G != 0) {
+            b[c] = bs[c];
+            continue;
+        }
+        const Pack w = *reinterpret_cast<const Pack *>(bs + c);
+#pragma unroll
+        for (int u = 0; u < G; ++u)
+            b[c + u] = w.v[u];
+    }
+#pragma unroll
+    for (int r = 0; r < TR; ++r) {
+#pragma unroll
+        for (int c = 0; c < TC; ++c) {
+            acc[r][c].x = fma(a[r].x, b[c].x, acc[r][c].x);
+            acc[r][c].y = fma(a[r].x, b[c].y, acc[r][c].y);
+        }
+#pragma unroll
+        for (int c = 0; c < TC; ++c) {
+            acc[r][c].x = fma(-a[r].y, b[c].y, acc[r][c].x);
+            acc[r][c].y = fma(a[r].y, b[c].x, acc[r][c].y);
+        }
+    }
+}
+
+// The eight warps' sums in warp order through `red` (MT x NT), then to C.
+template <typename T, int MT, int NT>
+__device__ __forceinline__ void SmallFinish(const typename C2<T>::type (&acc)[MT / 4][NT / 8],
+                                            typename C2<T>::type *red, typename C2<T>::type *C,
+                                            int64_t M, int64_t N, T scale)
+{
+    using V = typename C2<T>::type;
+    constexpr int TR = MT / 4, TC = NT / 8;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rg = lane >> 3, cg = lane & 7;
+    for (int w = 0; w < 8; ++w) {
+        if (warp == w) {
+#pragma unroll
+            for (int r = 0; r < TR; ++r)
+#pragma unroll
+                for (int c = 0; c < TC; ++c) {
+                    V &o = red[(rg * TR + r) * NT + cg * TC + c];
+                    if (w == 0)
+                        o = acc[r][c];
+                    else
+                        o = V{o.x + acc[r][c].x, o.y + acc[r][c].y};
+                }
+        }
+        __syncthreads();
+    }
+    for (int64_t e = tid; e < M * N; e += 256) {
+        const V v = red[(e / N) * NT + e % N];
+        C[e] = V{v.x * scale, v.y * scale};
+    }
+}
+
 // Products with a small output and a long k: M <= 16 and N <= 32, or M <= 32
 // and N <= 16, with k >= 2048 -- steps that close two large tensors down to a
 // few values, such as the 16 x 32 x 2^21 step of the reference's m10 network,
@@ -458,12 +541,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
     static_assert((TR == 1 || TR % 2 == 0) && (TC == 1 || TC % 2 == 0), "one or whole pairs");
     constexpr int kSmallKC = sizeof(T) == 4 ? 32 : 16;
     constexpr int NS = 2; // stages (three measured 5 % slower: occupancy, not latency, binds)
-    constexpr int G = 16 / sizeof(V); // elements per 16-byte shared-memory load
+    constexpr int G = 16 / sizeof(V); // elements per 16-byte shared-memory load: rows' padding
     // Copies per thread (the smallest tiles leave some threads without).
     constexpr int AP = (MT * kSmallKC + 255) / 256, BP = (NT * kSmallKC + 255) / 256;
-    struct alignas(16) Pack {
-        V v[G];
-    };
     __shared__ __align__(16) V As[NS][kSmallKC][MT + G];
     __shared__ __align__(16) V Bs[NS][kSmallKC][NT];
     __shared__ V red[MT * NT];
@@ -526,65 +606,158 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
         __syncthreads();
 #pragma unroll
         for (int kk = warp; kk < kSmallKC; kk += 8) {
-            V a[TR], b[TC];
-#pragma unroll
-            for (int r = 0; r < TR; r += G) {
-                if constexpr (TR % G != 0) {
-                    a[r] = As[st][kk][rg * TR + r];
-                    continue;
-                }
-                const Pack w = *reinterpret_cast<const Pack *>(&As[st][kk][rg * TR + r]);
-#pragma unroll
-                for (int u = 0; u < G; ++u)
-                    a[r + u] = w.v[u];
-            }
-#pragma unroll
-            for (int c = 0; c < TC; c += G) {
-                if constexpr (TC % G != 0) {
-                    b[c] = Bs[st][kk][cg * TC + c];
-                    continue;
-                }
-                const Pack w = *reinterpret_cast<const Pack *>(&Bs[st][kk][cg * TC + c]);
-#pragma unroll
-                for (int u = 0; u < G; ++u)
-                    b[c + u] = w.v[u];
-            }
-#pragma unroll
-            for (int r = 0; r < TR; ++r) {
-#pragma unroll
-                for (int c = 0; c < TC; ++c) {
-                    acc[r][c].x = fma(a[r].x, b[c].x, acc[r][c].x);
-                    acc[r][c].y = fma(a[r].x, b[c].y, acc[r][c].y);
-                }
-#pragma unroll
-                for (int c = 0; c < TC; ++c) {
-                    acc[r][c].x = fma(-a[r].y, b[c].y, acc[r][c].x);
-                    acc[r][c].y = fma(a[r].y, b[c].x, acc[r][c].y);
-                }
-            }
+            SmallMac<T, TR, TC>(acc, &As[st][kk][rg * TR], &Bs[st][kk][cg * TC]);
         }
         __syncthreads(); // the next load reuses this stage
         st ^= 1;
     }
-    for (int w = 0; w < 8; ++w) {
-        if (warp == w) {
+    SmallFinish<T, MT, NT>(acc, red, C, M, N, scale);
+}
+
+// Small outputs over a long k whose operands' axes are interleaved, read where
+// they lie: power-of-2 extents, so an element's place is a permutation of its
+// index bits. Transposing both operands first moves each twice more, which is
+// half of a closing step's time (16 x 32 x 2^21: two transposes 245 us of 499).
+//  * A tile is all of M and N and 2^kClosingLog k: the k bits lowest in A and
+//    lowest in B in turn, so both are read in runs of 64 bytes (complex64; a
+//    free axis among the low bits lengthens them). Tiles follow the next k
+//    bits up, so a CTA's consecutive tiles finish the lines around them.
+//  * A thread's copies stand at offsets fixed for the kernel from a base that
+//    moves by one addition per tile: from tile t to t + 1 it is the plan's
+//    step for the number of trailing ones of t.
+//  * In shared memory a k's row is padded by 16 bytes and every eight rows by
+//    16 more: copies along the low and along the high k bits then both spread
+//    over the banks.
+// The product is gemm_small_kernel's, over the k in the tiles' order, and bounds
+// it at 16 x 32 outputs (FMA issue; complex128 the FP64 pipe). 16 x 32 x 2^21
+// with both transposes before: 499 us, now 268; 4 x 8 x 2^21 reads 3.0 TB/s.
+constexpr int kClosingMaxBits = 32;
+template <typename T> constexpr int kClosingLog = sizeof(T) == 4 ? 6 : 5;
+
+struct ClosingSide {
+    uint32_t src[11]; // element bit (in the order of memory): its offset there,
+    uint32_t dst[11]; // ... and in a stage's rows
+    uint32_t tile[kClosingMaxBits]; // tile index bit: its offset
+    uint32_t step[kClosingMaxBits]; // from tile t to t + 1, by t's trailing ones
+};
+
+struct ClosingPlan {
+    ClosingSide a, b;
+    int tile_bits;
+};
+
+// A k's row in shared memory, of `width` elements.
+template <typename V> __host__ __device__ __forceinline__ int ClosingRow(int kk, int width)
+{
+    constexpr int G = 16 / sizeof(V);
+    return kk * (width + G) + (kk >> 3) * G;
+}
+
+// Where the element bits from `first` on of e place it (bits past the tile's
+// are zero in the plan).
+__host__ __device__ __forceinline__ void ClosingElement(const ClosingSide &p, int e, int first,
+                                                        int last, uint32_t &src, uint32_t &dst)
+{
+    src = dst = 0;
 #pragma unroll
-            for (int r = 0; r < TR; ++r)
-#pragma unroll
-                for (int c = 0; c < TC; ++c) {
-                    V &o = red[(rg * TR + r) * NT + cg * TC + c];
-                    if (w == 0)
-                        o = acc[r][c];
-                    else
-                        o = V{o.x + acc[r][c].x, o.y + acc[r][c].y};
-                }
+    for (int b = first; b < last; ++b)
+        if (e >> b & 1) {
+            src += p.src[b];
+            dst += p.dst[b];
         }
+}
+
+template <typename T, int MT, int NT> constexpr size_t ClosingShared()
+{
+    using V = typename C2<T>::type;
+    constexpr int KC = 1 << kClosingLog<T>, G = 16 / sizeof(V);
+    return 2 * (size_t)(KC * (MT + G) + KC / 8 * G + KC * (NT + G) + KC / 8 * G) * sizeof(V);
+}
+
+template <typename T, int MT, int NT>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
+    closing_kernel(const typename C2<T>::type *__restrict__ A,
+                   const typename C2<T>::type *__restrict__ B, typename C2<T>::type *__restrict__ C,
+                   int M, int N, uint32_t tiles, uint32_t per_cta, T scale,
+                   const __grid_constant__ ClosingPlan p)
+{
+    using V = typename C2<T>::type;
+    constexpr int TR = MT / 4, TC = NT / 8;
+    constexpr int KC = 1 << kClosingLog<T>, G = 16 / sizeof(V);
+    constexpr int AP = (MT * KC + 255) / 256, BP = (NT * KC + 255) / 256; // copies per thread
+    constexpr int kARows = KC * (MT + G) + KC / 8 * G, kBRows = KC * (NT + G) + KC / 8 * G;
+    static_assert(2 * (kARows + kBRows) >= MT * NT, "the sums reuse the stages");
+    extern __shared__ __align__(16) unsigned char closing_smem[];
+    V *const sm = reinterpret_cast<V *>(closing_smem); // two stages of A rows, B rows
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rg = lane >> 3, cg = lane & 7;
+    const uint32_t t0 = blockIdx.x * per_cta;
+    const uint32_t t1 = min(tiles, t0 + per_cta);
+
+    // Rows and columns past M and N stay zero.
+    for (int e = tid; e < 2 * (kARows + kBRows); e += 256)
+        sm[e] = V{0, 0};
+    // This thread's elements are tid + 256 q: the low bits once, q's from the plan.
+    uint32_t a_src, a_dst, b_src, b_dst;
+    ClosingElement(p.a, tid, 0, 8, a_src, a_dst);
+    ClosingElement(p.b, tid, 0, 8, b_src, b_dst);
+    const int a_count = M * KC, b_count = N * KC;
+    uint32_t a_base = 0, b_base = 0; // of the next tile to load
+    for (int b = 0; b < p.tile_bits; ++b)
+        if (t0 >> b & 1) {
+            a_base += p.a.tile[b];
+            b_base += p.b.tile[b];
+        }
+    auto load = [&](uint32_t t, int st) {
+        V *as = sm + st * (kARows + kBRows), *bs = as + kARows;
+#pragma unroll
+        for (int q = 0; q < AP; ++q)
+            if (tid + 256 * q < a_count) {
+                uint32_t src, dst;
+                ClosingElement(p.a, 256 * q, 8, 11, src, dst);
+                CpAsyncElem(as + a_dst + dst, A + (a_base + a_src + src), true);
+            }
+#pragma unroll
+        for (int q = 0; q < BP; ++q)
+            if (tid + 256 * q < b_count) {
+                uint32_t src, dst;
+                ClosingElement(p.b, 256 * q, 8, 11, src, dst);
+                CpAsyncElem(bs + b_dst + dst, B + (b_base + b_src + src), true);
+            }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        const int ones = __ffs(~t) - 1;
+        a_base += p.a.step[ones];
+        b_base += p.b.step[ones];
+    };
+
+    V acc[TR][TC];
+#pragma unroll
+    for (int r = 0; r < TR; ++r)
+#pragma unroll
+        for (int c = 0; c < TC; ++c)
+            acc[r][c] = V{0, 0};
+    __syncthreads(); // the zeros are in place
+    if (t0 < t1)
+        load(t0, 0);
+    int st = 0;
+    for (uint32_t t = t0; t < t1; ++t) {
+        if (t + 1 < t1)
+            load(t + 1, st ^ 1);
+        else
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory"); // all but the newest group
         __syncthreads();
+        const V *as = sm + st * (kARows + kBRows), *bs = as + kARows;
+#pragma unroll
+        for (int u = 0; u < KC / 8; ++u) {
+            const int kk = warp + 8 * u;
+            SmallMac<T, TR, TC>(acc, as + ClosingRow<V>(kk, MT) + rg * TR,
+                                bs + ClosingRow<V>(kk, NT) + cg * TC);
+        }
+        __syncthreads(); // the next load reuses this stage
+        st ^= 1;
     }
-    for (int64_t e = tid; e < M * N; e += 256) {
-        const V v = red[(e / N) * NT + e % N];
-        C[e] = V{v.x * scale, v.y * scale};
-    }
+    SmallFinish<T, MT, NT>(acc, sm, C + (int64_t)blockIdx.x * M * N, M, N, scale);
 }
 
 // Sums of the k ranges' partial results, accumulated in FP64: the partials
@@ -937,6 +1110,146 @@ int MultiplyVectorT(const typename C2<T>::type *A, const typename C2<T>::type *B
     return ReducePartials<T>(dst, C, batch * len, S, stream);
 }
 
+// The plan of closing_kernel, false where it does not apply: extents that are
+// not powers of 2, operands past 2^31 elements, outputs that SmallTile does not
+// take. Operands as ContractForm's (A permuted to (free, common), B to (common,
+// free)).
+bool PlanClosing(int a_rank, const uint64_t *a_shape, const int32_t *a_perm, int b_rank,
+                 const uint64_t *b_shape, const int32_t *b_perm, uint64_t m, uint64_t n, uint64_t k,
+                 int klog, ClosingPlan &p)
+{
+    int mt, nt;
+    const auto pow2 = [](uint64_t v) { return v > 0 && (v & (v - 1)) == 0; };
+    if (!pow2(m) || !pow2(n) || !pow2(k) || m > 32 || n > 32 || k > (1ull << 31) ||
+        m * k > (1ull << 31) || n * k > (1ull << 31))
+        return false;
+    SmallTile((int64_t)m, (int64_t)n, (int64_t)k, mt, nt);
+    if (!mt)
+        return false;
+    const auto log2of = [](uint64_t v) {
+        int l = 0;
+        while (v >>= 1)
+            ++l;
+        return l;
+    };
+    const int nk = log2of(k), nm = log2of(m), nn = log2of(n);
+    // Memory bit of every bit of the permuted index, lowest first.
+    int a_bit[64], b_bit[64];
+    const auto bits = [&](int rank, const uint64_t *shape, const int32_t *perm, int total,
+                          int *out) {
+        int place[64], at = 0, cnt = 0;
+        if (rank > 64)
+            return false;
+        for (int i = rank - 1; i >= 0; --i) {
+            if (!pow2(shape[i]))
+                return false;
+            place[i] = at;
+            at += log2of(shape[i]);
+        }
+        if (at != total)
+            return false;
+        for (int j = rank - 1; j >= 0; --j)
+            for (int u = 0; u < log2of(shape[perm[j]]); ++u)
+                out[cnt++] = place[perm[j]] + u;
+        return true;
+    };
+    if (!bits(a_rank, a_shape, a_perm, nm + nk, a_bit) ||
+        !bits(b_rank, b_shape, b_perm, nk + nn, b_bit))
+        return false;
+    const int *ak = a_bit, *am = a_bit + nk, *bn = b_bit, *bk = b_bit + nn;
+    // The tile's k bits: the lowest of A and of B in turn, the larger operand
+    // first.
+    bool in_tile[32] = {};
+    int chosen[8], count = 0;
+    for (int place = 0; place < 64 && count < klog; ++place)
+        for (int side = 0; side < 2; ++side)
+            for (int t = 0; t < nk && count < klog; ++t)
+                if (!in_tile[t] && ((side == 0) == (nn >= nm) ? bk[t] : ak[t]) == place) {
+                    in_tile[t] = true;
+                    chosen[count++] = t;
+                }
+    std::sort(chosen, chosen + klog, [&](int x, int y) { return ak[x] < ak[y]; });
+    int rest[32], nrest = 0;
+    for (int t = 0; t < nk; ++t)
+        if (!in_tile[t])
+            rest[nrest++] = t;
+    std::sort(rest, rest + nrest, [&](int x, int y) {
+        const int u = ak[x] < bk[x] ? ak[x] : bk[x], v = ak[y] < bk[y] ? ak[y] : bk[y];
+        return u != v ? u < v : x < y;
+    });
+    p = ClosingPlan{};
+    p.tile_bits = nrest;
+    const auto side = [&](ClosingSide &s, const int *kbit, const int *free_bit, int nfree,
+                          int across) {
+        std::vector<std::pair<int, int>> el; // memory bit, place in shared memory
+        for (int i = 0; i < klog; ++i) // additive over bits, as ClosingRow is
+            el.push_back({kbit[chosen[i]], klog == kClosingLog<float>
+                                               ? ClosingRow<float2>(1 << i, across)
+                                               : ClosingRow<double2>(1 << i, across)});
+        for (int u = 0; u < nfree; ++u)
+            el.push_back({free_bit[u], 1 << u});
+        std::sort(el.begin(), el.end());
+        for (size_t i = 0; i < el.size(); ++i) { // at most 6 + 5
+            s.src[i] = 1u << el[i].first;
+            s.dst[i] = (uint32_t)el[i].second;
+        }
+        uint32_t below = 0; // offsets that trailing ones leave
+        for (int i = 0; i < nrest; ++i) {
+            s.tile[i] = 1u << kbit[rest[i]];
+            s.step[i] = s.tile[i] - below;
+            below += s.tile[i];
+        }
+        s.step[nrest] = 0u - below; // past the last tile: not loaded
+    };
+    side(p.a, ak, am, nm, mt);
+    side(p.b, bk, bn, nn, nt);
+    return true;
+}
+
+template <typename T>
+int ClosingT(const ClosingPlan &p, const typename C2<T>::type *A, const typename C2<T>::type *B,
+             typename C2<T>::type *C, int64_t M, int64_t N, int64_t K, T scale, void *ws,
+             size_t ws_bytes, cudaStream_t stream)
+{
+    using V = typename C2<T>::type;
+    const int64_t tiles = K >> kClosingLog<T>;
+    // One wave; four tiles a CTA at least, or one where a tile keeps the FP64
+    // pipe busy for 20 us; the ranges' sums fit the workspace.
+    int64_t S = std::min<int64_t>((int64_t)SmCount() * (sizeof(T) == 4 ? 3 : 1),
+                                  sizeof(T) == 4 ? tiles / 4 : tiles);
+    S = std::min<int64_t>(S, ws ? (int64_t)(ws_bytes / (size_t)(M * N * (int64_t)sizeof(V))) : 1);
+    S = std::max<int64_t>(S, 1);
+    const int64_t per_cta = CeilDiv(tiles, S);
+    S = CeilDiv(tiles, per_cta);
+    V *dst = S > 1 ? (V *)ws : C;
+    int mt, nt;
+    SmallTile(M, N, K, mt, nt);
+    int rc = JETGPU_OK;
+    const auto launch = [&](auto kernel, size_t shared) {
+        // Enqueues nothing: a captured stream takes it too.
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)shared) != cudaSuccess)
+            rc = SetError(JETGPU_ERR_CUDA, "closing_kernel: shared memory limit not set");
+        else
+            kernel<<<(unsigned)S, 256, shared, stream>>>(A, B, dst, (int)M, (int)N,
+                                                         (uint32_t)tiles, (uint32_t)per_cta,
+                                                         scale, p);
+    };
+    if (mt == 4)
+        launch(closing_kernel<T, 4, 8>, ClosingShared<T, 4, 8>());
+    else if (mt == 8)
+        launch(closing_kernel<T, 8, 16>, ClosingShared<T, 8, 16>());
+    else if (mt == 16 && nt == 16)
+        launch(closing_kernel<T, 16, 16>, ClosingShared<T, 16, 16>());
+    else if (mt == 16)
+        launch(closing_kernel<T, 16, 32>, ClosingShared<T, 16, 32>());
+    else
+        launch(closing_kernel<T, 32, 16>, ClosingShared<T, 32, 16>());
+    if (rc || (rc = CheckLaunch("closing_kernel")) || S == 1)
+        return rc;
+    return ReducePartials<T>(dst, C, M * N, S, stream);
+}
+
 // Matrix product of `batch` pairs (strides sa, sb; 0 = shared), split over k
 // into the workspace when the tiles alone would leave SMs idle and the caller
 // supplied room for the partial sums (reduced in a fixed order).
@@ -1125,6 +1438,25 @@ int MultiplySingle(const void *A, const void *B, void *C, uint64_t m, uint64_t n
     return GemmT<float>((const float2 *)A, (const float2 *)B, (float2 *)C, 1, 0, 0, (int64_t)m,
                         (int64_t)n, (int64_t)k, (float)ldexp(1.0, scale_exp), workspace, bytes,
                         stream, S);
+}
+
+int ClosingContract(const void *A, int a_rank, const uint64_t *a_shape, const int32_t *a_perm,
+                    const void *B, int b_rank, const uint64_t *b_shape, const int32_t *b_perm,
+                    void *C, uint64_t m, uint64_t n, uint64_t k, int dtype, int scale_exp,
+                    void *workspace, size_t ws_bytes, cudaStream_t stream, bool &taken)
+{
+    ClosingPlan p;
+    const int klog = dtype == JETGPU_C128 ? kClosingLog<double> : kClosingLog<float>;
+    taken = PlanClosing(a_rank, a_shape, a_perm, b_rank, b_shape, b_perm, m, n, k, klog, p);
+    if (!taken)
+        return JETGPU_OK;
+    if (dtype == JETGPU_C128)
+        return ClosingT<double>(p, (const double2 *)A, (const double2 *)B, (double2 *)C,
+                                (int64_t)m, (int64_t)n, (int64_t)k, ldexp(1.0, scale_exp),
+                                workspace, ws_bytes, stream);
+    return ClosingT<float>(p, (const float2 *)A, (const float2 *)B, (float2 *)C, (int64_t)m,
+                           (int64_t)n, (int64_t)k, (float)ldexp(1.0, scale_exp), workspace,
+                           ws_bytes, stream);
 }
 
 size_t MultiplyPlainWorkspace(uint64_t m, uint64_t n, uint64_t k, int dtype)
