@@ -296,6 +296,15 @@ int jetgpu_contract_group(const jetgpu_group_task *tasks, int n_tasks, uint64_t 
                           int dtype, void *stream);
 
 /*
+ * jetgpu_contract_group where the task array and the offset tables were put on
+ * the device by a copy (or are otherwise complete when the kernel before this
+ * launch starts), not written by a kernel just before it: the launch may read
+ * them while that kernel still runs. Operands may be that kernel's output.
+ */
+int jetgpu_contract_group_uploaded(const jetgpu_group_task *tasks, int n_tasks,
+                                   uint64_t total_tiles, int dtype, void *stream);
+
+/*
  * jetgpu_contract without a workspace argument and without allocating: for
  * callers that cannot allocate device memory when they contract -- inside a
  * CUDA stream capture, where cudaMalloc is illegal; under a host's own fixed

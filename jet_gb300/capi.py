@@ -127,6 +127,7 @@ class GroupTask(ctypes.Structure):
 lib.jetgpu_group_tiles.restype = ctypes.c_uint64
 lib.jetgpu_group_tiles.argtypes = [ctypes.c_uint64, ctypes.c_uint64, ctypes.c_uint64]
 lib.jetgpu_contract_group.argtypes = [_vp, ctypes.c_int, ctypes.c_uint64, ctypes.c_int, _vp]
+lib.jetgpu_contract_group_uploaded.argtypes = lib.jetgpu_contract_group.argtypes
 lib.jetgpu_add.argtypes = [_vp, _vp, _vp, ctypes.c_uint64, ctypes.c_int, _vp]
 lib.jetgpu_conj.argtypes = [_vp, _vp, ctypes.c_uint64, ctypes.c_int, _vp]
 lib.jetgpu_slice_sum_f64.argtypes = [_vp, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int, _vp,
@@ -367,6 +368,14 @@ def contract_group_at(tasks_ptr: int, n_tasks: int, total_tiles: int, dtype_c: i
     """jetgpu_contract_group on a task array already on the device (its
     address, task count, summed jetgpu_group_tiles and dtype code)."""
     check(lib.jetgpu_contract_group(tasks_ptr, n_tasks, total_tiles, dtype_c, _stream(stream)))
+
+
+def contract_group_uploaded(tasks_ptr: int, n_tasks: int, total_tiles: int, dtype_c: int,
+                            stream=None) -> None:
+    """contract_group_at for tables that a copy from the host put there: the
+    launch may read them before the kernel ahead of it has ended."""
+    check(lib.jetgpu_contract_group_uploaded(tasks_ptr, n_tasks, total_tiles, dtype_c,
+                                             _stream(stream)))
 
 
 def split_tf32(x, shape, perm, rows, cols, pitch, planes, scale_exp=0, n_planes=4,

@@ -24,8 +24,15 @@
 // 7.5 us. Tiles of more work are staged in shared memory, 2 x 2 outputs a
 // thread. Whole k in one stage (64 of complex64) measured the same.
 // The launch uses programmatic stream serialisation, so that a chain of levels
-// overlaps each launch with the end of the one before: a gradient's replay
-// (53 grouped launches) 1,477 -> 1,459 us, 81 qutrit slices 4,498 -> 4,475 us.
+// overlaps each launch with the end of the one before. Where the tables were
+// uploaded by a copy (`uploaded`: the executors' launches), a launch reads them
+// -- tile scan, task, offsets: three of its five dependent loads -- before it
+// waits. Only operands need the kernel before, tables none: a launch starts
+// early behind a kernel, never behind a copy, and what came before that kernel
+// has ended. 16-qubit amplitude replay (13 levels) 124 -> 103 us, 720-angle
+// gradient (53 launches) 1,455 -> 1,375 us, 81 qutrit slices 4,494 -> 4,409 us
+// (without any early start 1,477 and 4,498). Tables that a kernel may have just
+// written are read after the wait.
 #include "common.cuh"
 
 namespace jetgpu {
@@ -61,19 +68,23 @@ template <typename V> __device__ __forceinline__ void GroupMac(V &acc, const V &
 template <typename T>
 __global__ void __launch_bounds__(kGThreads)
     group_contract_kernel(const jetgpu_group_task *__restrict__ tasks, int n_tasks,
-                          uint64_t total_tiles)
+                          uint64_t total_tiles, bool uploaded)
 {
     using V = typename V2<T>::type;
     __shared__ uint64_t first_tile[kMaxTasks + 1];
     __shared__ uint64_t warp_sum[kGThreads / 32];
     __shared__ V As[kGK][kGT + 1];
     __shared__ V Bs[kGK][kGT + 1];
-    // Every access to operands and outputs follows this wait for the kernel
-    // before; the next launch may start once every CTA is past it. The task
-    // table may be read earlier: a launch starts early only behind another
-    // grouped launch, which writes nothing but its outputs, and only once all
-    // that came before that one has ended.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // The wait for the kernel before: at the latest before the first operand.
+    bool waited = false;
+    const auto wait = [&]() {
+        if (!waited)
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+        waited = true;
+    };
+    if (!uploaded)
+        wait();
+    // The next launch may start once every CTA is past this.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // First tile of every task: thread t reads task t's tile count, then an
     // inclusive scan by warps and over the eight warp sums.
@@ -128,18 +139,26 @@ __global__ void __launch_bounds__(kGThreads)
                 const V *pb = B + q.b_col[n0 + j];
                 V acc{0, 0};
                 for (uint32_t k0 = 0; k0 < k; k0 += 8) {
+                    uint64_t ao[8], bo[8];
                     V av[8], bv[8];
 #pragma unroll
                     for (int u = 0; u < 8; ++u) { // past k: the last product's loads again
                         const uint32_t kk = min(k0 + u, k - 1);
-                        av[u] = pa[q.a_col[kk]];
-                        bv[u] = pb[q.b_row[kk]];
+                        ao[u] = q.a_col[kk];
+                        bo[u] = q.b_row[kk];
+                    }
+                    wait();
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        av[u] = pa[ao[u]];
+                        bv[u] = pb[bo[u]];
                     }
 #pragma unroll
                     for (int u = 0; u < 8; ++u)
                         if (k0 + u < k)
                             GroupMac(acc, av[u], bv[u]);
                 }
+                wait(); // no k: nothing was read
                 C[(m0 + i) * q.n + n0 + j] = acc;
             }
             continue;
@@ -154,14 +173,26 @@ __global__ void __launch_bounds__(kGThreads)
             // 32 x 32 of A (rows m0.., k k0..) and of B (k k0.., cols n0..):
             // 4 elements of each per thread, consecutive threads along k for A
             // and along n for B.
+            uint64_t ao[4], bo[4];
+            bool av[4], bv[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int idx = threadIdx.x + 256 * e;
                 const int rr = idx / kGK, cc = idx % kGK;
                 const uint64_t gi = m0 + rr, gk = k0 + cc;
-                As[cc][rr] = (gi < q.m && gk < q.k) ? A[q.a_row[gi] + q.a_col[gk]] : V{0, 0};
+                av[e] = gi < q.m && gk < q.k;
+                ao[e] = av[e] ? q.a_row[gi] + q.a_col[gk] : 0;
                 const uint64_t gk2 = k0 + rr, gj = n0 + cc;
-                Bs[rr][cc] = (gk2 < q.k && gj < q.n) ? B[q.b_row[gk2] + q.b_col[gj]] : V{0, 0};
+                bv[e] = gk2 < q.k && gj < q.n;
+                bo[e] = bv[e] ? q.b_row[gk2] + q.b_col[gj] : 0;
+            }
+            wait();
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int idx = threadIdx.x + 256 * e;
+                const int rr = idx / kGK, cc = idx % kGK;
+                As[cc][rr] = av[e] ? A[ao[e]] : V{0, 0};
+                Bs[rr][cc] = bv[e] ? B[bo[e]] : V{0, 0};
             }
             __syncthreads();
 #pragma unroll 8
@@ -186,22 +217,11 @@ __global__ void __launch_bounds__(kGThreads)
                     C[gi * q.n + gj] = acc[i][j];
             }
     }
+    wait(); // a launch never ends before the one that it started behind
 }
 
-} // namespace
-} // namespace jetgpu
-
-using namespace jetgpu;
-
-extern "C" {
-
-uint64_t jetgpu_group_tiles(uint64_t batch, uint64_t m, uint64_t n)
-{
-    return batch * ((m + kGT - 1) / kGT) * ((n + kGT - 1) / kGT);
-}
-
-int jetgpu_contract_group(const jetgpu_group_task *tasks, int n_tasks, uint64_t total_tiles,
-                          int dtype, void *stream)
+int LaunchGroup(const jetgpu_group_task *tasks, int n_tasks, uint64_t total_tiles, int dtype,
+                void *stream, bool uploaded)
 {
     NvtxRange range("jetgpu_contract_group");
     ClearError();
@@ -222,8 +242,32 @@ int jetgpu_contract_group(const jetgpu_group_task *tasks, int n_tasks, uint64_t 
     JETGPU_CUDA_TRY(cudaLaunchKernelEx(&cfg,
                                        dtype == JETGPU_C64 ? group_contract_kernel<float>
                                                            : group_contract_kernel<double>,
-                                       tasks, n_tasks, total_tiles));
+                                       tasks, n_tasks, total_tiles, uploaded));
     return CheckLaunch("group_contract_kernel");
+}
+
+} // namespace
+} // namespace jetgpu
+
+using namespace jetgpu;
+
+extern "C" {
+
+uint64_t jetgpu_group_tiles(uint64_t batch, uint64_t m, uint64_t n)
+{
+    return batch * ((m + kGT - 1) / kGT) * ((n + kGT - 1) / kGT);
+}
+
+int jetgpu_contract_group(const jetgpu_group_task *tasks, int n_tasks, uint64_t total_tiles,
+                          int dtype, void *stream)
+{
+    return LaunchGroup(tasks, n_tasks, total_tiles, dtype, stream, false);
+}
+
+int jetgpu_contract_group_uploaded(const jetgpu_group_task *tasks, int n_tasks,
+                                   uint64_t total_tiles, int dtype, void *stream)
+{
+    return LaunchGroup(tasks, n_tasks, total_tiles, dtype, stream, true);
 }
 
 } // extern "C"

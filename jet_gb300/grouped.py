@@ -102,7 +102,7 @@ class Group:
 
 
 def launch_group(group: Group) -> None:
-    capi.contract_group_at(group.ptr, len(group.tasks), group.tiles, group.dtype_code)
+    capi.contract_group_uploaded(group.ptr, len(group.tasks), group.tiles, group.dtype_code)
 
 
 class Schedule:

@@ -861,8 +861,8 @@ template <class T = std::complex<float>> class SlicedContractor {
                 Launch(steps_[item.steps[0]], st, prof);
                 continue;
             }
-            Gpu::Check(jetgpu_contract_group(item.tasks, (int)item.steps.size(), item.tiles, dt,
-                                             st),
+            Gpu::Check(jetgpu_contract_group_uploaded(item.tasks, (int)item.steps.size(),
+                                                      item.tiles, dt, st),
                        "grouped contraction");
             if (prof)
                 prof->Mark("group", item.steps.front(), item.steps.size(), 0, 0, 0);

@@ -586,9 +586,9 @@ template <class TensorType> class TaskBasedContractor {
             for (size_t it = 0; it < items.size(); ++it) {
                 const auto &item = items[it];
                 if (item.size() >= 2) {
-                    Gpu::Check(jetgpu_contract_group(task_dev + group_at[it].first,
-                                                     (int)item.size(), group_at[it].second, dt,
-                                                     st),
+                    Gpu::Check(jetgpu_contract_group_uploaded(task_dev + group_at[it].first,
+                                                              (int)item.size(),
+                                                              group_at[it].second, dt, st),
                                "grouped tiny steps (capture)");
                 }
                 else {
