@@ -629,7 +629,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
 //    16 more: copies along the low and along the high k bits then both spread
 //    over the banks.
 // The product is gemm_small_kernel's, over the k in the tiles' order, and bounds
-// it at 16 x 32 outputs (FMA issue; complex128 the FP64 pipe). 16 x 32 x 2^21
+// it at 16 x 32 outputs (issue of FMAs and the loads that feed a lane's 4 x 4
+// block, 32 TFLOP/s; complex128 the FP64 pipe). 16 x 32 x 2^21
 // with both transposes before: 499 us, now 268; 4 x 8 x 2^21 reads 3.0 TB/s.
 constexpr int kClosingMaxBits = 32;
 template <typename T> constexpr int kClosingLog = sizeof(T) == 4 ? 6 : 5;
