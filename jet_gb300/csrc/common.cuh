@@ -131,6 +131,12 @@ inline uint64_t SplitPitchAlign(SplitFormat f) { return f == SplitFormat::kTf32 
 // words followed by their lo words, 128 bytes a block, so that one TMA row
 // brings both. For columns in whole blocks.
 inline uint64_t SplitPairWords(SplitFormat f) { return f == SplitFormat::kTf32 ? 16 : 32; }
+// A TMA coordinate is a 32-bit int and counts words: k in planar rows, 2 k in
+// paired ones. Past its range a box would read zeros, and its terms be lost
+// without an error. The ranges of a cut k together span up to one stage (32 k)
+// per range more than k, at most a range per SM: 2^14 words leave room for that.
+constexpr uint64_t kMaxCutK = (1ull << 31) - (1ull << 14);
+constexpr uint64_t kMaxPairedK = kMaxCutK / 2;
 
 // FP16 split: an operand whose largest magnitude has binary exponent e_max
 // (jetgpu_max_exponent; -1000 when all zero) is multiplied by 2^s before the

@@ -76,9 +76,10 @@ SplitLayout LayoutFor(int precision, uint64_t k, double work, int variant = -1,
     l.a_planes = algo == JETGPU_ALGO_3M ? 6 : 4;
     l.b_planes = (algo == JETGPU_ALGO_3M || l.variant == 1) ? 6 : 4;
     l.group_m = group_m;
-    // The default loops read paired planes where k is whole blocks; the same
-    // bytes either way.
-    l.paired = l.variant == 0 && algo == JETGPU_ALGO_4M && k % SplitPairWords(l.fmt) == 0;
+    // The default loops read paired planes where k is whole blocks and their
+    // words stay in a coordinate's range; the same bytes either way.
+    l.paired = l.variant == 0 && algo == JETGPU_ALGO_4M && k % SplitPairWords(l.fmt) == 0 &&
+               k <= kMaxPairedK;
     return l;
 }
 

@@ -543,6 +543,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const uint32_t fb = SmemAddr(&full_bar[s]);
                 MbarArriveExpectTx(fb, kStageBytes);
                 const uint32_t base = SmemAddr(smem + s * kStageBytes);
+                // Words; below 2^31 (kMaxPairedK, kMaxCutK).
                 const int k0 = ((total_ktiles > 0 ? bz * ktiles : 0) + kt) * kBK *
                                (kPaired ? 2 : 1);
 #pragma unroll
@@ -1265,6 +1266,7 @@ int LaunchSplitProduct(const void *a_planes, int a_batched, const void *b_planes
     JETGPU_REQUIRE(kpitch >= (paired ? 2 : 1) * k && kpitch % SplitPitchAlign(fmt) == 0,
                    "bad k pitch");
     JETGPU_REQUIRE(!paired || k % SplitPairWords(fmt) == 0, "paired planes need whole blocks");
+    JETGPU_REQUIRE(!paired || k <= kMaxPairedK, "k too large for paired planes");
     JETGPU_REQUIRE(((uintptr_t)a_planes % 16) == 0 && ((uintptr_t)b_planes % 16) == 0,
                    "planes must be 16-byte aligned");
     JETGPU_REQUIRE(((n + kBN - 1) / kBN) * ((m + kBM - 1) / kBM) <= 0x7fffffffull,
@@ -1354,7 +1356,7 @@ int TcSplits(uint64_t m, uint64_t n, uint64_t k, SplitFormat fmt)
     const uint64_t tiles = ((n + kBN - 1) / kBN) * ((m + kBM - 1) / kBM);
     const uint64_t stage_k = fmt == SplitFormat::kTf32 ? 16 : 32;
     const uint64_t stages = (k + stage_k - 1) / stage_k;
-    if (tiles == 0 || m * n * sizeof(float2) > (32ull << 20))
+    if (tiles == 0 || m * n * sizeof(float2) > (32ull << 20) || k > kMaxCutK)
         return 1;
     uint64_t s = (uint64_t)SmCount() / tiles;
     s = std::min(s, k / 256);
