@@ -231,8 +231,9 @@ int GemmSplitPlanarBatched(const void *a_planes, int a_batched, const void *b_pl
 // whole), and the bytes of partial sums they need: see gemm_tc.cu.
 int TcSplits(uint64_t m, uint64_t n, uint64_t k, SplitFormat fmt);
 
-// out[i] = sum over s < splits of part[s * len + i], in order, rounded once
-// (complex64).
+// out[i] = sum over s < splits of part[s * len + i], in order (complex64):
+// within (splits - 1)^2 2^-48 of the sum of magnitudes before one rounding, and
+// finite wherever the sum is (gemm_simt.cu).
 int SumPartials(const void *part, void *out, uint64_t len, uint64_t splits, cudaStream_t stream);
 
 // Workspace bytes of a (batched) contraction in `precision` (JETGPU_PREC_TUNED:

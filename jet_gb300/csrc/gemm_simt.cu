@@ -818,8 +818,11 @@ __global__ void reduce_partials_warp(const typename C2<T>::type *__restrict__ pa
 // The sums of a jetgpu_contract product's k ranges, complex64, in range order.
 // FP64 adds and conversions bound the kernel above on this GPU (2^18 outputs of
 // nine ranges 24 us, their 19 MB in L2): here the running sum is a pair of
-// FP32 values, the second holding the exact rounding errors of the first's
-// adds (Knuth's two-sum), so a sum is rounded once at the end, as in FP64.
+// FP32 values, the second adding up the exact rounding errors of the first's
+// adds (Knuth's two-sum). Those adds of errors round too: S ranges are off by
+// at most (S - 1)^2 2^-48 of the sum of their magnitudes before the last
+// rounding. The range is FP32's, so a sum that leaves it on the way, or meets
+// an infinity or NaN, is taken again in FP64.
 struct PairSum {
     float s = 0, e = 0;
     __device__ __forceinline__ void add(float x)
@@ -829,8 +832,6 @@ struct PairSum {
         e += (s - (t - b)) + (x - b);
         s = t;
     }
-    // An infinite or NaN sum has no error to add.
-    __device__ __forceinline__ float value() const { return isfinite(s) ? s + e : s; }
 };
 
 __global__ void __launch_bounds__(256)
@@ -857,7 +858,17 @@ __global__ void __launch_bounds__(256)
             re.add(v.x);
             im.add(v.y);
         }
-        out[i] = make_float2(re.value(), im.value());
+        float2 r = make_float2(re.s + re.e, im.s + im.e);
+        if (!isfinite(re.s) || !isfinite(im.s)) { // once there, a sum stays there
+            double x = 0, y = 0;
+#pragma unroll 1
+            for (s = 0; s < S; ++s) {
+                x += part[s * len + i].x;
+                y += part[s * len + i].y;
+            }
+            r = make_float2((float)x, (float)y);
+        }
+        out[i] = r;
     }
 }
 
