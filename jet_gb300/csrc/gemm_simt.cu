@@ -872,6 +872,17 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// Few outputs of many ranges take a warp each (reduce_partials_warp, FP64, one
+// warp per CTA: FP64 adds bound it): a thread that walks its ranges alone waits
+// out a memory latency per four of them. Thread against warp, us back to back:
+// 289 outputs 18 / 6 at 256 ranges, 66 / 10 at 1,024; 2,048 outputs 8.2 / 6.2 at
+// 64; 4,096 outputs 10.3 / 10.3 at 128, 18 / 14 at 256; 8,192 outputs 35 / 44 at
+// 512.
+inline bool SumByWarps(uint64_t len, uint64_t ranges)
+{
+    return ranges >= 64 && (len <= 2048 || (len <= 4096 && ranges >= 256));
+}
+
 // Sums S partial results of `len` elements each into out (a fixed order).
 template <typename T>
 int ReducePartials(const typename C2<T>::type *part, typename C2<T>::type *out, int64_t len,
@@ -976,16 +987,26 @@ inline double TileClocks(const GemmTile &t, int64_t M, int64_t N, int64_t z)
     return std::max(t.alone, (double)per_sm * t.shared);
 }
 
+// Split-k factor of a batched product (fixed: the slices of a sliced network
+// keep their bits whatever tile a launch gets): GemmSplits over tiles of 128
+// (complex64) or 64 (complex128) rows, 32 when M <= 32, and 64 columns.
+template <typename T> int64_t BatchedSplits(int64_t batch, int64_t M, int64_t N, int64_t K)
+{
+    const int64_t bm = M <= 32 ? 32 : (sizeof(T) == 4 ? 128 : 64);
+    return GemmSplits(CeilDiv(M, bm) * CeilDiv(N, 64) * batch, batch, K,
+                      batch * M * N * (int64_t)(2 * sizeof(T)));
+}
+
 // k ranges of one product (jetgpu_contract): products of few tiles leave SMs
 // idle, so k is cut while the busiest SM then finishes sooner, adding the
 // ranges' sums (a launch, and their bytes through L2) included. At least 64 k
 // a range, and none below 256: steps of k <= 64 add in one order everywhere
-// (grouped launches and skinny kernels give the same bits).
-constexpr int64_t kSingleMinK = 256;
+// (grouped launches and skinny kernels give the same bits). At most 1,024 of
+// complex64: past that a CTA's own start and end cost more than the fuller last
+// wave saves (2 x 40 outputs, k = 2^18: 1,024 ranges 115 us, 4,096 149).
+constexpr int64_t kSingleMinK = 256, kSingleRanges = 1024;
 constexpr double kReduceClocks = 6000.0; // a launch and its latency
 constexpr double kReduceBytes = 2000.0;  // partial sums per clock
-
-template <typename T> int64_t SingleSplits(int64_t M, int64_t N, int64_t K);
 
 inline int PickTileC64(int64_t M, int64_t N, int64_t z)
 {
@@ -1004,7 +1025,7 @@ template <typename T> int64_t SingleSplits(int64_t M, int64_t N, int64_t K)
     double least = 0;
     for (int64_t S = 1; K / S >= kSingleMinK / 4; S *= 2) {
         const double bytes = (double)S * M * N * 2 * sizeof(T);
-        if (S > 1 && bytes > (double)(32 << 20))
+        if (S > 1 && (bytes > (double)(32 << 20) || (sizeof(T) == 4 && S > kSingleRanges)))
             break;
         const GemmTile &t = sizeof(T) == 4 ? kTilesC64[PickTileC64(M, N, S)] : kTileC128;
         const double clocks = TileClocks(t, M, N, S) * (double)CeilDiv(K, S) +
@@ -1015,16 +1036,6 @@ template <typename T> int64_t SingleSplits(int64_t M, int64_t N, int64_t K)
         }
     }
     return best;
-}
-
-// Split-k factor of a batched product (fixed: the slices of a sliced network
-// keep their bits whatever tile a launch gets): GemmSplits over tiles of 128
-// (complex64) or 64 (complex128) rows, 32 when M <= 32, and 64 columns.
-template <typename T> int64_t BatchedSplits(int64_t batch, int64_t M, int64_t N, int64_t K)
-{
-    const int64_t bm = M <= 32 ? 32 : (sizeof(T) == 4 ? 128 : 64);
-    return GemmSplits(CeilDiv(M, bm) * CeilDiv(N, 64) * batch, batch, K,
-                      batch * M * N * (int64_t)(2 * sizeof(T)));
 }
 
 // Split-k factor for the vector kernels: enough CTAs to fill the GPU, with at
@@ -1408,6 +1419,11 @@ int MultiplyPlainBatched(const void *A, const void *B, void *C, uint64_t batch, 
 
 int SumPartials(const void *part, void *out, uint64_t len, uint64_t splits, cudaStream_t stream)
 {
+    if (SumByWarps(len, splits)) {
+        reduce_partials_warp<float><<<GridFor(len, 32), 32, 0, stream>>>(
+            (const float2 *)part, (float2 *)out, (int64_t)len, (int64_t)splits);
+        return CheckLaunch("reduce_partials_warp");
+    }
     sum_partials_kernel<<<GridFor((len + 255) / 256, 8), 256, 0, stream>>>(
         (const float2 *)part, (float2 *)out, (int64_t)len, (int64_t)splits);
     return CheckLaunch("sum_partials_kernel");
