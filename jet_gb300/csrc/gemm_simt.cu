@@ -1003,7 +1003,9 @@ template <typename T> int64_t BatchedSplits(int64_t batch, int64_t M, int64_t N,
 // a range, and none below 256: steps of k <= 64 add in one order everywhere
 // (grouped launches and skinny kernels give the same bits). At most 1,024 of
 // complex64: past that a CTA's own start and end cost more than the fuller last
-// wave saves (2 x 40 outputs, k = 2^18: 1,024 ranges 115 us, 4,096 149).
+// wave saves (2 x 40 outputs, k = 2^18: 1,024 ranges 115 us, 4,096 149). Never fewer
+// than a batch of one gets, whose sums would otherwise be the closer ones: an
+// output of four ranges of 839 k was 1.5 times as far off as one of nine of 373.
 constexpr int64_t kSingleMinK = 256, kSingleRanges = 1024;
 constexpr double kReduceClocks = 6000.0; // a launch and its latency
 constexpr double kReduceBytes = 2000.0;  // partial sums per clock
@@ -1021,21 +1023,24 @@ template <typename T> int64_t SingleSplits(int64_t M, int64_t N, int64_t K)
 {
     if (K < kSingleMinK || SmCount() < 1)
         return 1;
-    int64_t best = 1;
+    const int64_t first = BatchedSplits<T>(1, M, N, K);
+    int64_t best = 0;
     double least = 0;
     for (int64_t S = 1; K / S >= kSingleMinK / 4; S *= 2) {
         const double bytes = (double)S * M * N * 2 * sizeof(T);
         if (S > 1 && (bytes > (double)(32 << 20) || (sizeof(T) == 4 && S > kSingleRanges)))
             break;
+        if (S < first)
+            continue;
         const GemmTile &t = sizeof(T) == 4 ? kTilesC64[PickTileC64(M, N, S)] : kTileC128;
         const double clocks = TileClocks(t, M, N, S) * (double)CeilDiv(K, S) +
                               (S > 1 ? kReduceClocks + bytes / kReduceBytes : 0.0);
-        if (S == 1 || clocks < least) {
+        if (best == 0 || clocks < least) {
             best = S;
             least = clocks;
         }
     }
-    return best;
+    return best > 0 ? best : first;
 }
 
 // Split-k factor for the vector kernels: enough CTAs to fill the GPU, with at
