@@ -187,8 +187,15 @@ int jetgpu_multiply(const void *A, const void *B, void *C, uint64_t m,
  * |scale_a + scale_b| <= 126.
  * scale_a, scale_b: power-of-two exponents applied exactly to A and B before
  * the product (C = (2^scale_a A)(2^scale_b B)); 0 for none.
- * workspace: caller-owned device scratch of at least
- * jetgpu_contract_workspace_size(...) bytes (may be NULL when that is 0).
+ * workspace: caller-owned device scratch of jetgpu_contract_workspace_size(...)
+ * bytes (may be NULL when that is 0). In that much, k of a product with few
+ * output tiles is cut into ranges whose sums are added at the end (plain forms
+ * from k = 256, tensor-core forms from k = 512). Less is accepted down to what
+ * the contraction cannot do without, jetgpu_contract_batched_workspace_size of
+ * a batch of 1 (ALGO_4M): k is then cut as that entry point cuts it. The
+ * order of additions, and so a result's last bits, depends on which of the two
+ * the workspace holds, never on its contents. JETGPU_PREC_TUNED always runs as
+ * with the smaller size.
  * Products with one side at most 16 wide and k <= 64 (a gate on a large
  * tensor) read A and B in place through the permutations and need none.
  */
@@ -314,8 +321,8 @@ int jetgpu_contract_group_uploaded(const jetgpu_group_task *tasks, int n_tasks,
  *
  * Scratch comes from one 32 MiB device array inside the library (every GPU
  * that loads the library holds it until the process exits); a contraction
- * whose jetgpu_contract_workspace_size exceeds
- * jetgpu_contract_noalloc_max_scratch() is rejected with
+ * that cannot do with jetgpu_contract_noalloc_max_scratch() bytes
+ * (jetgpu_contract_batched_workspace_size of a batch of 1) is rejected with
  * JETGPU_ERR_WORKSPACE. The first call on each device looks up the array's
  * device address (cudaGetSymbolAddress) with that device current; make that
  * first call before any stream capture. All calls share the one array: calls
@@ -324,7 +331,9 @@ int jetgpu_contract_group_uploaded(const jetgpu_group_task *tasks, int n_tasks,
  * address is cached per device for the life of the process: after a
  * cudaDeviceReset the module is loaded again and the array may move, so a
  * process that resets a device must not call this entry point on it again.
- * Arguments and results are those of jetgpu_contract.
+ * Arguments are those of jetgpu_contract, and so are results, bit for bit
+ * where jetgpu_contract_workspace_size is within that limit; beyond it k may be
+ * cut less, which moves the last bits.
  */
 int jetgpu_contract_noalloc(const void *A, int a_rank, const uint64_t *a_shape,
                             const int32_t *a_perm, const void *B, int b_rank,

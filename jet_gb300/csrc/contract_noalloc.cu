@@ -65,7 +65,8 @@ int jetgpu_contract_noalloc(const void *A, int a_rank, const uint64_t *a_shape,
                             int algo, int scale_a, int scale_b, void *stream)
 {
     jetgpu::ClearError();
-    // What the contraction cannot do without; a cut of k takes room that is left.
+    // What the contraction cannot do without; the sums of a cut k take room that
+    // is left.
     const size_t need = jetgpu::ContractWorkspace(1, a_rank, a_shape, a_perm, 0, b_rank, b_shape,
                                                   b_perm, 0, m, n, k, dtype, precision);
     if (need > jetgpu::kScratchBytes)
@@ -75,8 +76,13 @@ int jetgpu_contract_noalloc(const void *A, int a_rank, const uint64_t *a_shape,
                 " bytes of scratch, more than the " + std::to_string(jetgpu::kScratchBytes) +
                 " bytes the allocation-free entry point holds; use jetgpu_contract with a "
                 "caller-provided workspace");
+    // jetgpu_contract asks for more where it cuts k, also where an uncut product
+    // needs nothing: it gets the scratch whenever it asks.
+    const size_t asked = jetgpu_contract_workspace_size_algo(a_rank, a_shape, a_perm, b_rank,
+                                                             b_shape, b_perm, m, n, k, dtype,
+                                                             precision, algo);
     void *scratch = nullptr;
-    if (need > 0) {
+    if (need > 0 || asked > 0) {
         const int rc = jetgpu::ScratchAddress(&scratch);
         if (rc != JETGPU_OK)
             return rc;
@@ -86,7 +92,7 @@ int jetgpu_contract_noalloc(const void *A, int a_rank, const uint64_t *a_shape,
     // to be cleared between calls.
     return jetgpu_contract(A, a_rank, a_shape, a_perm, B, b_rank, b_shape, b_perm, C, m, n, k,
                            dtype, precision, algo, scale_a, scale_b, scratch,
-                           need > 0 ? jetgpu::kScratchBytes : 0, stream);
+                           scratch ? jetgpu::kScratchBytes : 0, stream);
 }
 
 } // extern "C"
