@@ -974,8 +974,11 @@ constexpr GemmTile kTilesC64[] = {
     {64, 32, 122, 105}, // 4 x 2, 256 threads
     {32, 64, 128, 112}, // 2 x 4
     {32, 32, 83, 61},   // 2 x 2
+    // Short k only (PickTileC64): no clocks.
+    {64, 64, 0, 0}, // 4 x 4, 256 threads, 8 k a slice
+    {32, 64, 0, 0}, // 4 x 4, 128 threads, 8 k a slice
 };
-constexpr int kNumTilesC64 = sizeof(kTilesC64) / sizeof(kTilesC64[0]);
+constexpr int kLongTilesC64 = 6;
 constexpr GemmTile kTileC128 = {32, 32, 2100, 2100};
 
 inline int64_t CeilDiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
@@ -1010,12 +1013,29 @@ constexpr int64_t kSingleMinK = 256, kSingleRanges = 1024;
 constexpr double kReduceClocks = 6000.0; // a launch and its latency
 constexpr double kReduceBytes = 2000.0;  // partial sums per clock
 
-inline int PickTileC64(int64_t M, int64_t N, int64_t z)
+// The clocks are per k, so short products, which load and store more than they
+// multiply, are picked apart. A slice of 16 k is mostly zeros for k = 2..8, and the
+// 32-row tiles' two or three CTAs per SM keep too little in flight. us with the
+// clocks' pick / with the pick here:
+//   20 x 300,000 outputs   k = 2 47 / 23, 16 50 / 37, 32 79 / 65, 65 158 / 137,
+//                          128 240 / 236
+//   64 of 27 x 81          k = 3 3.4 / 2.6, 27 4.6 / 4.3 (81 8.8 / 8.1)
+//   500 x 500              k = 2 3.1 / 2.6, 32 4.1 / 4.1 (64 6.0 / 6.4)
+//   65,536 x 33            k <= 8 12.6 / 11.3, 16 16.8 / 16.8
+//   4000 x 4096            k <= 8 37.5 / 37.8
+// Launches of at most one 32 x 32 tile per SM have nothing to gain.
+inline int PickTileC64(int64_t M, int64_t N, int64_t K, int64_t z)
 {
     int best = 0;
-    for (int i = 1; i < kNumTilesC64; ++i)
+    for (int i = 1; i < kLongTilesC64; ++i)
         if (TileClocks(kTilesC64[i], M, N, z) < TileClocks(kTilesC64[best], M, N, z))
             best = i;
+    if (K <= 8 && best == 0)
+        return 6;
+    const int64_t tiles = CeilDiv(M, 32) * CeilDiv(N, 32) * z;
+    if ((best == 4 || best == 5) && tiles > (int64_t)SmCount() &&
+        K <= (tiles > 8 * (int64_t)SmCount() ? 96 : 32))
+        return 7;
     return best;
 }
 
@@ -1032,8 +1052,9 @@ template <typename T> int64_t SingleSplits(int64_t M, int64_t N, int64_t K)
             break;
         if (S < first)
             continue;
-        const GemmTile &t = sizeof(T) == 4 ? kTilesC64[PickTileC64(M, N, S)] : kTileC128;
-        const double clocks = TileClocks(t, M, N, S) * (double)CeilDiv(K, S) +
+        const int64_t kchunk = CeilDiv(K, S);
+        const GemmTile &t = sizeof(T) == 4 ? kTilesC64[PickTileC64(M, N, kchunk, S)] : kTileC128;
+        const double clocks = TileClocks(t, M, N, S) * (double)kchunk +
                               (S > 1 ? kReduceClocks + bytes / kReduceBytes : 0.0);
         if (best == 0 || clocks < least) {
             best = S;
@@ -1322,7 +1343,7 @@ int GemmT(const typename C2<T>::type *A, const typename C2<T>::type *B, typename
                           ? BatchedSplits<T>(batch, M, N, K)
                           : 1;
     const int64_t kchunk = (K + S - 1) / S;
-    const int tile = sizeof(T) == 4 ? PickTileC64(M, N, batch * S) : 0;
+    const int tile = sizeof(T) == 4 ? PickTileC64(M, N, kchunk, batch * S) : 0;
     const GemmTile t = sizeof(T) == 4 ? kTilesC64[tile] : kTileC128;
     const int64_t tiles = CeilDiv(M, t.bm) * CeilDiv(N, t.bn);
     JETGPU_REQUIRE(tiles <= 0x7fffffffLL && batch * S <= 65535, "product too large for one launch");
@@ -1351,8 +1372,14 @@ int GemmT(const typename C2<T>::type *A, const typename C2<T>::type *B, typename
         case 4:
             launch(gemm_kernel<float, 2, 4, 16, 16, 16, 2>, 256);
             break;
-        default:
+        case 5:
             launch(gemm_kernel<float, 2, 2, 16, 16, 16, 3>, 256);
+            break;
+        case 6:
+            launch(gemm_kernel<float, 4, 4, 16, 16, 8, 3>, 256);
+            break;
+        default:
+            launch(gemm_kernel<float, 4, 4, 16, 8, 8, 5>, 128);
         }
     }
     int rc = CheckLaunch("gemm_kernel");
