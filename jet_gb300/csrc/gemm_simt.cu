@@ -834,6 +834,41 @@ struct PairSum {
     }
 };
 
+// Ranges [s, last) of output i, in order, the loads of U at once.
+template <int U>
+__device__ __forceinline__ void AddRanges(const float2 *__restrict__ part, int64_t len, int64_t i,
+                                          int64_t s, int64_t last, PairSum &re, PairSum &im)
+{
+    for (; s + U <= last; s += U) {
+        float2 v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            v[u] = part[(s + u) * len + i];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            re.add(v[u].x);
+            im.add(v[u].y);
+        }
+    }
+    if constexpr (U > 1)
+        AddRanges<U / (U > 4 ? 2 : 4)>(part, len, i, s, last, re, im);
+}
+
+__device__ __forceinline__ float2 SumOfRanges(const float2 *__restrict__ part, int64_t len,
+                                              int64_t i, int64_t S, const PairSum &re,
+                                              const PairSum &im)
+{
+    if (isfinite(re.s) && isfinite(im.s)) // once not finite, a sum stays so
+        return make_float2(re.s + re.e, im.s + im.e);
+    double x = 0, y = 0;
+#pragma unroll 1
+    for (int64_t s = 0; s < S; ++s) {
+        x += part[s * len + i].x;
+        y += part[s * len + i].y;
+    }
+    return make_float2((float)x, (float)y);
+}
+
 __global__ void __launch_bounds__(256)
     sum_partials_kernel(const float2 *__restrict__ part, float2 *__restrict__ out, int64_t len,
                         int64_t S)
@@ -841,46 +876,46 @@ __global__ void __launch_bounds__(256)
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len;
          i += (int64_t)gridDim.x * blockDim.x) {
         PairSum re, im;
-        int64_t s = 0;
-        for (; s + 4 <= S; s += 4) {
-            float2 v[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                v[u] = part[(s + u) * len + i];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                re.add(v[u].x);
-                im.add(v[u].y);
-            }
-        }
-        for (; s < S; ++s) {
-            const float2 v = part[s * len + i];
-            re.add(v.x);
-            im.add(v.y);
-        }
-        float2 r = make_float2(re.s + re.e, im.s + im.e);
-        if (!isfinite(re.s) || !isfinite(im.s)) { // once there, a sum stays there
-            double x = 0, y = 0;
-#pragma unroll 1
-            for (s = 0; s < S; ++s) {
-                x += part[s * len + i].x;
-                y += part[s * len + i].y;
-            }
-            r = make_float2((float)x, (float)y);
-        }
-        out[i] = r;
+        AddRanges<4>(part, len, i, 0, S, re, im);
+        out[i] = SumOfRanges(part, len, i, S, re, im);
     }
 }
 
-// Few outputs of many ranges take a warp each (reduce_partials_warp, FP64, one
-// warp per CTA: FP64 adds bound it): a thread that walks its ranges alone waits
-// out a memory latency per four of them. Thread against warp, us back to back:
-// 289 outputs 18 / 6 at 256 ranges, 66 / 10 at 1,024; 2,048 outputs 8.2 / 6.2 at
-// 64; 4,096 outputs 10.3 / 10.3 at 128, 18 / 14 at 256; 8,192 outputs 35 / 44 at
-// 512.
-inline bool SumByWarps(uint64_t len, uint64_t ranges)
+// From kManyRanges ranges on, where one thread per output waits out a memory
+// latency per four of them: the warps of a CTA each add a share of the ranges of
+// 32 outputs, the first warp their sums in order. us back to back, a thread per
+// output / a warp of FP64 adds / these: 289 outputs of 256 ranges 18 / 6 / 4, of
+// 1,024 66 / 10 / 8; 4,096 outputs of 256 18 / 14 / 4; 65,536 of 64 8 / 98 / 10.
+constexpr uint64_t kManyRanges = 64;
+constexpr int kManyWarps = 16;
+
+__global__ void __launch_bounds__(32 * kManyWarps)
+    sum_many_kernel(const float2 *__restrict__ part, float2 *__restrict__ out, int64_t len,
+                    int64_t S)
 {
-    return ranges >= 64 && (len <= 2048 || (len <= 4096 && ranges >= 256));
+    __shared__ float4 sums[kManyWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t per = (S + kManyWarps - 1) / kManyWarps;
+    for (int64_t i0 = (int64_t)blockIdx.x * 32; i0 < len; i0 += (int64_t)gridDim.x * 32) {
+        const int64_t i = i0 + lane;
+        PairSum re, im;
+        if (i < len)
+            AddRanges<8>(part, len, i, min(S, warp * per), min(S, (warp + 1) * per), re, im);
+        sums[warp][lane] = make_float4(re.s, re.e, im.s, im.e);
+        __syncthreads();
+        if (warp == 0 && i < len) {
+#pragma unroll
+            for (int w = 1; w < kManyWarps; ++w) {
+                const float4 q = sums[w][lane];
+                re.add(q.x);
+                re.e += q.y;
+                im.add(q.z);
+                im.e += q.w;
+            }
+            out[i] = SumOfRanges(part, len, i, S, re, im);
+        }
+        __syncthreads(); // the sums are read
+    }
 }
 
 // Sums S partial results of `len` elements each into out (a fixed order).
@@ -1451,10 +1486,10 @@ int MultiplyPlainBatched(const void *A, const void *B, void *C, uint64_t batch, 
 
 int SumPartials(const void *part, void *out, uint64_t len, uint64_t splits, cudaStream_t stream)
 {
-    if (SumByWarps(len, splits)) {
-        reduce_partials_warp<float><<<GridFor(len, 32), 32, 0, stream>>>(
+    if (splits >= kManyRanges) {
+        sum_many_kernel<<<GridFor((len + 31) / 32, 4), 32 * kManyWarps, 0, stream>>>(
             (const float2 *)part, (float2 *)out, (int64_t)len, (int64_t)splits);
-        return CheckLaunch("reduce_partials_warp");
+        return CheckLaunch("sum_many_kernel");
     }
     sum_partials_kernel<<<GridFor((len + 255) / 256, 8), 256, 0, stream>>>(
         (const float2 *)part, (float2 *)out, (int64_t)len, (int64_t)splits);
