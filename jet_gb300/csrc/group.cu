@@ -54,8 +54,12 @@ template <> struct V2<double> {
 
 // Most multiply-adds of a tile that goes through the tables directly (8 k of a
 // full 32 x 32 tile), and its longest k.
+// And its most outputs: with 4 a thread, complex64 is slower than staged (one
+// 32 x 32 x 2..8 task 5.4 us, staged 5.0; 6 of 256 x 256 x 1 8.4 and 7.9), where
+// complex128, whose padding costs FP64 adds, takes 12 us and staged 36.
 constexpr uint64_t kFlatWork = 8192;
 constexpr uint64_t kFlatK = 64;
+template <typename T> constexpr uint32_t kFlatOutputs = sizeof(T) == 4 ? 512 : 1024;
 
 template <typename V> __device__ __forceinline__ void GroupMac(V &acc, const V &a, const V &b)
 {
@@ -131,7 +135,7 @@ __global__ void __launch_bounds__(kGThreads)
         V *C = static_cast<V *>(q.C) + b * q.m * q.n;
         const uint32_t rows = (uint32_t)min(q.m - m0, (uint64_t)kGT);
         const uint32_t cols = (uint32_t)min(q.n - n0, (uint64_t)kGT);
-        if (q.k <= kFlatK && rows * cols * q.k <= kFlatWork) {
+        if (q.k <= kFlatK && rows * cols <= kFlatOutputs<T> && rows * cols * q.k <= kFlatWork) {
             const uint32_t k = (uint32_t)q.k;
             for (uint32_t e = threadIdx.x; e < rows * cols; e += kGThreads) {
                 const uint32_t i = e / cols, j = e - i * cols;
