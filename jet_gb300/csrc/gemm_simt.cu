@@ -230,10 +230,6 @@ template <typename T> struct KahanSum {
     }
 };
 
-// Groups of four products whose loads a thread of the vector kernels issues
-// at once (32 eight-byte or 16 sixteen-byte loads).
-template <typename T> constexpr int kVectorGroups = sizeof(T) == 4 ? 4 : 2;
-
 // y[b, m] (+ partial s) = sum_{k in chunk s} A_b[m, k] x_b[k]. A CTA of 8
 // warps covers `rows` rows (8, 4, 2 or 1) with 8 / rows warps per row, which
 // interleave the row's k chunk, so few rows still keep every warp streaming.
@@ -263,32 +259,12 @@ __global__ void __launch_bounds__(256)
     if (m < M) {
         // Four products per compensated add: four loads in flight per thread
         // and a quarter of the compensation work (the sum of four products
-        // carries one rounding of the plain FMA chain).
+        // carries one rounding of the plain FMA chain). Several groups' loads at
+        // once, as in gemv_cols_kernel, cost more registers than they hide
+        // here: complex64 100 x 3000 6.6 us with one group, 7.1 with two, 8.1
+        // with four, 4096 x 4096 26, 30 and 32.
         const int64_t step = wpr * 32;
         int64_t k = k_begin + part * 32 + lane;
-        // Several such groups' loads at once: a split's few rows leave most
-        // SMs with one CTA, which would wait out a memory latency per group.
-        constexpr int G = kVectorGroups<T>;
-        for (; k + (4 * G - 1) * step < k_end; k += 4 * G * step) {
-            V a[4 * G], xv[4 * G];
-#pragma unroll
-            for (int u = 0; u < 4 * G; ++u) {
-                a[u] = A[m * K + k + u * step];
-                xv[u] = x[k + u * step];
-            }
-#pragma unroll
-            for (int g = 0; g < G; ++g) {
-                T re = a[4 * g].x * xv[4 * g].x - a[4 * g].y * xv[4 * g].y;
-                T im = a[4 * g].x * xv[4 * g].y + a[4 * g].y * xv[4 * g].x;
-#pragma unroll
-                for (int u = 4 * g + 1; u < 4 * g + 4; ++u) {
-                    re = fma(a[u].x, xv[u].x, fma(-a[u].y, xv[u].y, re));
-                    im = fma(a[u].x, xv[u].y, fma(a[u].y, xv[u].x, im));
-                }
-                sr.add(re);
-                si.add(im);
-            }
-        }
         for (; k + 3 * step < k_end; k += 4 * step) {
             V a[4], xv[4];
 #pragma unroll
@@ -340,7 +316,12 @@ __global__ void __launch_bounds__(256)
 // consecutive elements of B's rows. `cols` = 1 is the dot product. Batch b =
 // blockIdx.z (strides sa, sb; 0 = shared). Partial s of column (b, n) lands at
 // out[(s * batch + b) * N + n].
-template <typename T>
+// G: groups of four products whose loads a thread issues at once. A thread of
+// a narrow B waits out a memory latency per group: two groups, us against one
+// and four, complex64 1 x 256 x 1024 55 (139, 71), 1 x 4096 x 4096 151 (375, 211),
+// 81 of 1 x 243 x 243 18.7 (35.0, 19.4); complex128 1 x 4096 x 4096 499 (565).
+// complex128 dot products take one: k = 2^22 84 (two 126).
+template <typename T, int G>
 __global__ void __launch_bounds__(256)
     gemv_cols_kernel(const typename C2<T>::type *__restrict__ x,
                      const typename C2<T>::type *__restrict__ B,
@@ -361,10 +342,10 @@ __global__ void __launch_bounds__(256)
     out += (s * gridDim.z + b) * N;
     KahanSum<T> sr, si;
     if (n < N) {
-        // Four products per compensated add, several groups' loads at once
+        // Four products per compensated add, the loads of G groups at once
         // (see gemv_rows_kernel).
         int64_t k = k_begin + tk;
-        constexpr int G = kVectorGroups<T>;
+        if constexpr (G > 1)
         for (; k + (4 * G - 1) * (int64_t)tk_count < k_end; k += 4 * G * (int64_t)tk_count) {
             V a[4 * G], v[4 * G];
 #pragma unroll
@@ -1182,12 +1163,16 @@ int MultiplyVectorT(const typename C2<T>::type *A, const typename C2<T>::type *B
     const int64_t kchunk = (K + S - 1) / S;
     V *dst = S > 1 ? (V *)ws : C;
     const dim3 grid((unsigned)blocks, (unsigned)S, (unsigned)batch);
+    const auto launch = [&](auto kernel) {
+        kernel<<<grid, 256, 0, stream>>>(A, B, dst, N == 1 && M > 1 ? M : N, K, kchunk, scale,
+                                         sa, sb, per_cta);
+    };
     if (N == 1 && M > 1)
-        gemv_rows_kernel<T><<<grid, 256, 0, stream>>>(A, B, dst, M, K, kchunk, scale, sa, sb,
-                                                      per_cta);
+        launch(gemv_rows_kernel<T>);
+    else if (sizeof(T) == 8 && per_cta == 1)
+        launch(gemv_cols_kernel<T, 1>);
     else
-        gemv_cols_kernel<T><<<grid, 256, 0, stream>>>(A, B, dst, N, K, kchunk, scale, sa, sb,
-                                                      per_cta);
+        launch(gemv_cols_kernel<T, 2>);
     int rc = CheckLaunch(N == 1 && M > 1 ? "gemv_rows_kernel" : "gemv_cols_kernel");
     if (rc || S == 1)
         return rc;
