@@ -303,10 +303,16 @@ int jetgpu_contract_group(const jetgpu_group_task *tasks, int n_tasks, uint64_t 
                           int dtype, void *stream);
 
 /*
- * jetgpu_contract_group where the task array and the offset tables were put on
- * the device by a copy (or are otherwise complete when the kernel before this
- * launch starts), not written by a kernel just before it: the launch may read
- * them while that kernel still runs. Operands may be that kernel's output.
+ * jetgpu_contract_group for task arrays and offset tables that are on the device
+ * already: the launch may read them before the work ahead of it in the stream
+ * has ended. Grouped launches, and jetgpu_contract calls of a few outputs, that
+ * follow each other in a stream form a run in which each may start while all of
+ * the earlier ones, and the kernel ahead of the run, still execute. The array
+ * and tables must be complete when that kernel starts, and stay unchanged until this
+ * launch has ended: copied before it or directly before the run in the same
+ * stream, or complete before the host makes the calls. Never written by a
+ * kernel of the run or by the one ahead of it (jetgpu_contract_group takes
+ * those). Operands may be outputs of any of them.
  */
 int jetgpu_contract_group_uploaded(const jetgpu_group_task *tasks, int n_tasks,
                                    uint64_t total_tiles, int dtype, void *stream);

@@ -372,8 +372,8 @@ def contract_group_at(tasks_ptr: int, n_tasks: int, total_tiles: int, dtype_c: i
 
 def contract_group_uploaded(tasks_ptr: int, n_tasks: int, total_tiles: int, dtype_c: int,
                             stream=None) -> None:
-    """contract_group_at for tables that a copy from the host put there: the
-    launch may read them before the kernel ahead of it has ended."""
+    """contract_group_at for tables that are complete already (copied before, see
+    jetgpu.h): the launch may read them before the work ahead of it has ended."""
     check(lib.jetgpu_contract_group_uploaded(tasks_ptr, n_tasks, total_tiles, dtype_c,
                                              _stream(stream)))
 

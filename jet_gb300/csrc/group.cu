@@ -27,12 +27,23 @@
 // overlaps each launch with the end of the one before. Where the tables were
 // uploaded by a copy (`uploaded`: the executors' launches), a launch reads them
 // -- tile scan, task, offsets: three of its five dependent loads -- before it
-// waits. Only operands need the kernel before, tables none: a launch starts
-// early behind a kernel, never behind a copy, and what came before that kernel
-// has ended. 16-qubit amplitude replay (13 levels) 124 -> 103 us, 720-angle
-// gradient (53 launches) 1,455 -> 1,375 us, 81 qutrit slices 4,494 -> 4,409 us
-// (without any early start 1,477 and 4,498). Tables that a kernel may have just
-// written are read after the wait.
+// waits. 16-qubit amplitude replay (13 levels) 124 -> 103 us, 720-angle gradient
+// (53 launches) 1,455 -> 1,375 us, 81 qutrit slices 4,494 -> 4,409 us (without any
+// early start 1,477 and 4,498). Tables that a kernel may have just written are
+// read after the wait.
+//  * What a launch may read before its wait: these launches and skinny.cu's tiny
+//    steps let the next one start before they wait themselves, so in an unbroken
+//    run of them a launch may start while any earlier one of the run, and the
+//    kernel that the run follows, still execute. Its tables must have been
+//    complete when that kernel started: copied before it, or directly before the
+//    run (a launch starts early behind a kernel only), or waited for by the host,
+//    as the executors do once after they upload theirs.
+//  * The wait ends when the launch before has ended, which waited for the one
+//    before it: everything earlier has ended too, and its writes are visible.
+//  * What an earlier launch of the run may write (operands; task arrays that were
+//    not uploaded) is read by plain loads: no pointer to it is const
+//    __restrict__, whose loads may take the non-coherent path, which is for memory
+//    that nobody writes while the kernel runs.
 #include "common.cuh"
 
 namespace jetgpu {
@@ -70,9 +81,8 @@ template <typename V> __device__ __forceinline__ void GroupMac(V &acc, const V &
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kGThreads)
-    group_contract_kernel(const jetgpu_group_task *__restrict__ tasks, int n_tasks,
-                          uint64_t total_tiles, bool uploaded)
+__device__ __forceinline__ void GroupContract(const jetgpu_group_task *tasks, int n_tasks,
+                                              uint64_t total_tiles, bool uploaded)
 {
     using V = typename V2<T>::type;
     __shared__ uint64_t first_tile[kMaxTasks + 1];
@@ -224,6 +234,24 @@ __global__ void __launch_bounds__(kGThreads)
     wait(); // a launch never ends before the one that it started behind
 }
 
+// The task array may be the output of the kernel before.
+template <typename T>
+__global__ void __launch_bounds__(kGThreads)
+    group_contract_kernel(const jetgpu_group_task *tasks, int n_tasks, uint64_t total_tiles)
+{
+    GroupContract<T>(tasks, n_tasks, total_tiles, false);
+}
+
+// The task array is complete: its fields are read again where they are used (64
+// registers in complex64; kept, 94).
+template <typename T>
+__global__ void __launch_bounds__(kGThreads)
+    group_uploaded_kernel(const jetgpu_group_task *__restrict__ tasks, int n_tasks,
+                          uint64_t total_tiles)
+{
+    GroupContract<T>(tasks, n_tasks, total_tiles, true);
+}
+
 int LaunchGroup(const jetgpu_group_task *tasks, int n_tasks, uint64_t total_tiles, int dtype,
                 void *stream, bool uploaded)
 {
@@ -243,11 +271,13 @@ int LaunchGroup(const jetgpu_group_task *tasks, int n_tasks, uint64_t total_tile
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    JETGPU_CUDA_TRY(cudaLaunchKernelEx(&cfg,
-                                       dtype == JETGPU_C64 ? group_contract_kernel<float>
-                                                           : group_contract_kernel<double>,
-                                       tasks, n_tasks, total_tiles, uploaded));
-    return CheckLaunch("group_contract_kernel");
+    JETGPU_CUDA_TRY(cudaLaunchKernelEx(
+        &cfg,
+        dtype == JETGPU_C64
+            ? (uploaded ? group_uploaded_kernel<float> : group_contract_kernel<float>)
+            : (uploaded ? group_uploaded_kernel<double> : group_contract_kernel<double>),
+        tasks, n_tasks, total_tiles));
+    return CheckLaunch(uploaded ? "group_uploaded_kernel" : "group_contract_kernel");
 }
 
 } // namespace

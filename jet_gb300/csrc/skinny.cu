@@ -294,15 +294,16 @@ constexpr int kSkTiny = 4096;
 
 template <typename T, bool BigIsA>
 __global__ void __launch_bounds__(kSkThreads)
-    skinny_tiny_kernel(const typename C2<T>::type *__restrict__ big,
-                       const typename C2<T>::type *__restrict__ small,
-                       typename C2<T>::type *__restrict__ C,
+    skinny_tiny_kernel(const typename C2<T>::type *big, const typename C2<T>::type *small,
+                       typename C2<T>::type *C,
                        const __grid_constant__ SkinnyParams p, T scale)
 {
     using V = typename C2<T>::type;
     // Launched with programmatic stream serialisation: the launch may begin
     // while the previous kernel of the stream finishes, and the next one may
-    // start launching now (it waits for this one).
+    // start launching now (it waits for this one). The operands may be that kernel's
+    // output, written while this one already runs: plain pointers, because loads
+    // through const __restrict__ ones may take the non-coherent path (group.cu).
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t b = blockIdx.y;
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
