@@ -80,9 +80,9 @@ template <typename V> __device__ __forceinline__ void GroupMac(V &acc, const V &
     acc.y = fma(a.y, b.x, acc.y);
 }
 
-template <typename T>
+template <typename T, bool kUploaded>
 __device__ __forceinline__ void GroupContract(const jetgpu_group_task *tasks, int n_tasks,
-                                              uint64_t total_tiles, bool uploaded)
+                                              uint64_t total_tiles)
 {
     using V = typename V2<T>::type;
     __shared__ uint64_t first_tile[kMaxTasks + 1];
@@ -96,7 +96,7 @@ __device__ __forceinline__ void GroupContract(const jetgpu_group_task *tasks, in
             asm volatile("griddepcontrol.wait;" ::: "memory");
         waited = true;
     };
-    if (!uploaded)
+    if (!kUploaded)
         wait();
     // The next launch may start once every CTA is past this.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -133,7 +133,20 @@ __device__ __forceinline__ void GroupContract(const jetgpu_group_task *tasks, in
         for (int step = kMaxTasks / 2; step > 0; step >>= 1)
             if (t + step < n_tasks && first_tile[t + step] <= g)
                 t += step;
-        const jetgpu_group_task &q = tasks[t];
+        const jetgpu_group_task *task = tasks + t;
+        if constexpr (!kUploaded) {
+            // Its own copy: read by plain loads, the fields would be read again
+            // after every store.
+            __shared__ jetgpu_group_task copy;
+            constexpr int kWords = sizeof(jetgpu_group_task) / sizeof(uint64_t);
+            __syncthreads(); // the tile before has been read
+            if (threadIdx.x < kWords)
+                reinterpret_cast<uint64_t *>(&copy)[threadIdx.x] =
+                    reinterpret_cast<const uint64_t *>(task)[threadIdx.x];
+            __syncthreads();
+            task = &copy;
+        }
+        const jetgpu_group_task &q = *task;
         const uint64_t local = g - first_tile[t];
         const uint64_t tiles_n = (q.n + kGT - 1) / kGT;
         const uint64_t tiles_mn = ((q.m + kGT - 1) / kGT) * tiles_n;
@@ -239,7 +252,7 @@ template <typename T>
 __global__ void __launch_bounds__(kGThreads)
     group_contract_kernel(const jetgpu_group_task *tasks, int n_tasks, uint64_t total_tiles)
 {
-    GroupContract<T>(tasks, n_tasks, total_tiles, false);
+    GroupContract<T, false>(tasks, n_tasks, total_tiles);
 }
 
 // The task array is complete: its fields are read again where they are used (64
@@ -249,7 +262,7 @@ __global__ void __launch_bounds__(kGThreads)
     group_uploaded_kernel(const jetgpu_group_task *__restrict__ tasks, int n_tasks,
                           uint64_t total_tiles)
 {
-    GroupContract<T>(tasks, n_tasks, total_tiles, true);
+    GroupContract<T, true>(tasks, n_tasks, total_tiles);
 }
 
 int LaunchGroup(const jetgpu_group_task *tasks, int n_tasks, uint64_t total_tiles, int dtype,
