@@ -460,7 +460,9 @@ def run_ours(args, rank, world, local_rank):
     # DRAM bytes (read + write) per launch of the product at this size: a
     # constant taken from one ncu capture of this workload, not measured in
     # this run (CUDA events cannot count DRAM bytes); null where none was taken.
-    traffic = {"tf32x3": 14.77e9, "bf16x3": 7.67e9}.get(head)
+    # The stages timed here hand planar operands over, so they run the planar
+    # main loops (kernel_v); jetgpu_contract runs the paired ones on its own.
+    traffic = {"tf32x3": 18.34e9, "bf16x3": 7.92e9, "fp16x3": 8.62e9}.get(head)
     form_names = {"tf32x3": "TF32x3 4M (tcgen05 kind::tf32, hi/lo split, 3 products)",
                   "bf16x3": "BF16x3 4M (tcgen05 kind::f16 on BF16, hi/lo split, 3 products)",
                   "fp16x3": "FP16x3 4M (tcgen05 kind::f16 on FP16 hi/lo of power-of-two "

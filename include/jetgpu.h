@@ -50,7 +50,9 @@ extern "C" {
                                 ~2^-22 truncation per product (TF32x3's) */
 #define JETGPU_PREC_TUNED 5  /* per contraction key, the fastest of FP32, TF32X3 (either main
                                 loop) and FP16X3 (either tile order), timed on first use
-                                (jetgpu_autotune_*);
+                                (jetgpu_autotune_*), each as jetgpu_contract_batched runs it
+                                (without jetgpu_contract's further cuts of k and its closing
+                                steps read in place, with which AUTO can be the faster form);
                                 AUTO for small steps and for keys first met during capture */
 
 /* Complex product algorithms for the tensor-core form. */
